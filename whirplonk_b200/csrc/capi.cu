@@ -220,7 +220,7 @@ whirgpu_status acquire_workspace(whirgpu_ctx* c, uint64_t n, const whirgpu_param
 void prepare_lde_tables(whirgpu_ctx* c, const ProofPlan& plan) {
     for (const CommitBuffers& cb : plan.commits) {
         const uint64_t room = c->budget ? (c->budget > c->allocated ? c->budget - c->allocated : 0) : ~0ull;
-        lde_tables_prepare(c->lde_tables, cb.logN, cb.logX, c->tw.tw_hi, c->tw.tw_lo, c->stream, room);
+        lde_tables_prepare(c->lde_tables, cb.logN, cb.logX, cb.depth * cb.ncomp, c->tw.tw_hi, c->tw.tw_lo, c->stream, room);
     }
 }
 
@@ -323,6 +323,8 @@ whirgpu_status whirgpu_ctx_create(int device, uint64_t hbm_budget, whirgpu_ctx**
     WG_CUDA(nullptr, cudaMemcpy(c->tw.tw_hi, hi.data(), hi.size() * 8, cudaMemcpyHostToDevice), "upload");
     WG_CUDA(nullptr, cudaMemcpy(c->tw.tw_lo, lo.data(), lo.size() * 8, cudaMemcpyHostToDevice), "upload");
     c->tw.lde = &c->lde_tables;
+    WG_CUDA(nullptr, cudaHostAlloc(&c->lde_err, sizeof(uint32_t), cudaHostAllocMapped), "cudaHostAlloc");
+    *c->lde_err = 0;
     *out = c.release();
     return WHIRGPU_OK;
 }
@@ -346,6 +348,7 @@ void whirgpu_ctx_destroy(whirgpu_ctx* c) {
     cudaFree(c->tw.tw_hi);
     cudaFree(c->tw.tw_lo);
     lde_tables_free(c->lde_tables);
+    if (c->lde_err) cudaFreeHost(c->lde_err);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->mle_scratch) cudaFree(c->mle_scratch);
     if (c->kscratch) cudaFree(c->kscratch);

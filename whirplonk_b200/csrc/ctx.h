@@ -99,6 +99,7 @@ struct whirgpu_ctx {
     uint64_t ws_allocations = 0, ws_evictions = 0;  // workspaces allocated / freed to make room
     wg::DeviceTables tw;
     wg::LdeTables lde_tables;  // inter-pass twiddle factors of the LDE splits in use (tw.lde)
+    uint32_t* lde_err = nullptr;  // pinned, mapped: error bits of the kernel-level encoder calls
     std::string err;
     // Workspaces by plan shape: the schedule, hash engine, vector layout, field
     // degree and domain-separator length, serialised (plan_key).

@@ -6,8 +6,8 @@
 // every value is kept canonical in [0, p).  The 64x64 product is formed with
 // mul.lo/mul.hi and reduced with the sparse-prime identities
 //   2^64 == 2^32 - 1,   2^96 == -1   (mod p).
-// This is exact integer work for the CUDA cores; there is nothing for the
-// tensor cores here.
+// This is exact integer work for the CUDA cores (the encoder's DFTs also run
+// as 8-bit contractions on the tensor cores, k_dft8.cu).
 #pragma once
 #include <cstdint>
 

@@ -19,6 +19,7 @@
 #include <atomic>
 #include <map>
 #include <mutex>
+#include <set>
 #include <tuple>
 #include <utility>
 
@@ -658,18 +659,24 @@ bool lde_plan_valid(const LdePlan& p) {
 
 static std::mutex g_plan_mu;
 static std::map<u32, LdePlan> g_plans;  // key logN << 8 | logX
+static std::set<u32> g_forced;          // keys of forced plans
 static std::atomic<u32> g_plan_epoch{0};
 
-void lde_install_plan(u32 logX, const LdePlan& p) {
+void lde_install_plan(u32 logX, const LdePlan& p, bool forced) {
     std::lock_guard<std::mutex> lk(g_plan_mu);
     const u32 key = p.logN << 8 | logX;
+    g_forced.erase(key);
     if (p.npass == 0) g_plans.erase(key);
-    else g_plans[key] = p;
+    else {
+        g_plans[key] = p;
+        if (forced) g_forced.insert(key);
+    }
     ++g_plan_epoch;
 }
 void lde_clear_plans() {
     std::lock_guard<std::mutex> lk(g_plan_mu);
     g_plans.clear();
+    g_forced.clear();
     ++g_plan_epoch;
 }
 u32 lde_plan_epoch() { return g_plan_epoch.load(); }
@@ -816,10 +823,25 @@ int launch_lde_plan(const LdeArgs& L, const LdePlan& pl, cudaStream_t st) {
     return 0;
 }
 
+// Whether the shape runs as 8-bit contractions: from 2^20 codeword words up.
+// The two contraction passes have a floor of 19-30 us (their constants and one
+// tile's round trip); below 2^20 words the butterfly passes take 9-25 us.
+// Measured (us, contraction / butterfly): 48 planes 2^12 -> 2^14 31 / 25,
+// 16 planes 2^14 -> 2^16 29 / 33, 16 planes 2^20 -> 2^22 923 / 1658, 48 planes
+// 2^16 -> 2^21 1157 / 1846, 48 planes 2^12 -> 2^20 435 / 752.
+static bool use_dft8(u32 logN, u32 logX, u32 planes) {
+    if (((u64)planes << logN) < (1ull << 20) || !dft8_applicable(logN, logX, planes)) return false;
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    return !g_forced.count(logN << 8 | logX);
+}
+
 int launch_lde(const LdeArgs& L, cudaStream_t st) {
     u32 lm = 0;
     while ((1ull << lm) < L.m) ++lm;
     const u32 logX = L.logN > lm ? L.logN - lm : 0;
+    if (L.logN == lm + logX && L.m == 1ull << lm && L.tables && use_dft8(L.logN, logX, L.planes) &&
+        L.tables->get(L.logN, dft8_first_bits(L.logN, logX)))
+        return launch_dft8(L, logX, st);
     return launch_lde_plan(L, plan_lde(L.logN, logX), st);
 }
 
@@ -831,17 +853,16 @@ __global__ void k_pass_table(u64* tab, u32 logNs, u32 logS, const u64* hi, const
         tab[k] = twiddle((k >> logS) * (k & mask), logNs, hi, lo);
 }
 
-long long lde_tables_prepare_plan(LdeTables& t, const LdePlan& pl, const u64* tw_hi, const u64* tw_lo,
-                                  cudaStream_t st, u64 room) {
-    if (!lde_plan_valid(pl)) return 0;
+// Tables of the first `n` pass boundaries of a 2^logNs transform (radices logR).
+static long long build_tables(LdeTables& t, u32 logNs, const u32* logRs, u32 n, const u64* tw_hi, const u64* tw_lo,
+                              cudaStream_t st, u64 room) {
     u64* made[3] = {};
     u32 keys[3] = {};
     int nmade = 0;
     long long bytes = 0;
-    u32 logNs = pl.logN;
-    for (u32 s = 0; s + 1 < pl.npass; ++s) {
-        const u32 logR = pl.logR[s];
-        const u32 key = logNs * (TW_STAGE_LOG + 1) + logR;
+    for (u32 s = 0; s < n; ++s) {
+        const u32 logR = logRs[s];
+        const u32 key = logNs * LdeTables::STRIDE + logR;
         const size_t sz = (size_t)8 << logNs;
         if (t.tab[key].load() == nullptr && logNs <= LdeTables::MAX_LOG && (u64)bytes + sz <= room) {
             u64* p = nullptr;
@@ -868,15 +889,25 @@ long long lde_tables_prepare_plan(LdeTables& t, const LdePlan& pl, const u64* tw
         u64* expect = nullptr;
         if (!t.tab[keys[k]].compare_exchange_strong(expect, made[k])) {  // built meanwhile by another thread
             cudaFree(made[k]);
-            bytes -= (long long)((size_t)8 << (keys[k] / (TW_STAGE_LOG + 1)));
+            bytes -= (long long)((size_t)8 << (keys[k] / LdeTables::STRIDE));
         }
     }
     return bytes;
 }
 
-long long lde_tables_prepare(LdeTables& t, u32 logN, u32 logX, const u64* tw_hi, const u64* tw_lo, cudaStream_t st,
-                             u64 room) {
+long long lde_tables_prepare_plan(LdeTables& t, const LdePlan& pl, const u64* tw_hi, const u64* tw_lo,
+                                  cudaStream_t st, u64 room) {
+    return lde_plan_valid(pl) ? build_tables(t, pl.logN, pl.logR, pl.npass - 1, tw_hi, tw_lo, st, room) : 0;
+}
+
+long long lde_tables_prepare(LdeTables& t, u32 logN, u32 logX, u32 planes, const u64* tw_hi, const u64* tw_lo,
+                             cudaStream_t st, u64 room) {
     if (logN > TW_LOG) return 0;
+    if (logN <= LdeTables::MAX_LOG && use_dft8(logN, logX, planes)) {
+        const u32 r = dft8_first_bits(logN, logX);
+        const long long b = build_tables(t, logN, &r, 1, tw_hi, tw_lo, st, room);
+        if (b < 0 || t.get(logN, r)) return b;
+    }
     return lde_tables_prepare_plan(t, plan_lde(logN, logX), tw_hi, tw_lo, st, room);
 }
 
@@ -897,7 +928,7 @@ int lde_prepare() {
                 return -1;
             for (u32 lw = 0; lw <= 6 && lw <= l; ++lw) pipe_occupancy(mb, l, lw);
         }
-    return 0;
+    return dft8_prepare();
 }
 
 }  // namespace wg

@@ -98,7 +98,15 @@ LdeArgs lde_args(whirgpu_ctx* c, const u64* src, u64 m, u32 planes, u32 logN, u6
     L.tw_hi = c->tw.tw_hi;
     L.tw_lo = c->tw.tw_lo;
     L.tables = &c->lde_tables;
+    L.err = c->lde_err;
     return L;
+}
+
+// The inter-pass tables of the form launch_lde takes for a shape.
+void prepare_shape_tables(whirgpu_ctx* c, u32 logN, u32 logX, u32 planes) {
+    std::lock_guard<std::recursive_mutex> lk(c->cache_mu);
+    const uint64_t room = c->budget ? (c->budget > c->allocated ? c->budget - c->allocated : 0) : ~0ull;
+    lde_tables_prepare(c->lde_tables, logN, logX, planes, c->tw.tw_hi, c->tw.tw_lo, c->stream, room);
 }
 
 // The inter-pass tables of `pl` (kernel-level calls run outside graph capture).
@@ -127,7 +135,7 @@ whirgpu_status whirgpu_rs_encode(whirgpu_ctx* c, const uint64_t* d_vectors, size
     const u64 planes = (u64)count << log_depth;
     if (planes > 65535) return fail(c, WHIRGPU_E_INVALID, "too many planes");
     const u32 logN = log_len - log_depth + log_expansion;
-    prepare_plan_tables(c, plan_lde(logN, log_expansion));
+    prepare_shape_tables(c, logN, log_expansion, (u32)planes);
     const LdeArgs L = lde_args(c, d_vectors, 1ull << (log_len - log_depth), (u32)planes, logN, d_tmp, d_planes);
     if (launch_lde(L, c->stream) != 0) return fail(c, WHIRGPU_E_INVALID, "LDE launch");
     const cudaError_t e = cudaGetLastError();
@@ -143,7 +151,7 @@ whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* c, const uint64_t* vectors, 
     const u32 logN = log_len - log_depth + log_expansion;
     const u64 N = 1ull << logN;
     const u64 in_words = count << log_len;
-    prepare_plan_tables(c, plan_lde(logN, log_expansion));
+    prepare_shape_tables(c, logN, log_expansion, (u32)planes);
     const u64 node_words = (2 * N) * 8;  // 32-bit words of one tree's node array
     const size_t bytes = (location == WHIRGPU_INPUT_DEVICE ? 0 : in_words * 8) + 2 * planes * N * 8 +
                          count * node_words * 4 + 256;
@@ -175,7 +183,9 @@ whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* c, const uint64_t* vectors, 
         if (e != cudaSuccess) return cuda_fail(c, e, "root copy");
     }
     const cudaError_t e = cudaStreamSynchronize(c->stream);
-    return e == cudaSuccess ? WHIRGPU_OK : cuda_fail(c, e, "rs_commit");
+    if (e != cudaSuccess) return cuda_fail(c, e, "rs_commit");
+    if (*(volatile uint32_t*)c->lde_err) return fail(c, WHIRGPU_E_DEVICE, "encoder wait ran out");
+    return WHIRGPU_OK;
 }
 
 // ---- pass-plan autotuner --------------------------------------------------
@@ -268,7 +278,7 @@ whirgpu_status whirgpu_ntt_autotune(whirgpu_ctx* c, uint32_t log_n, uint32_t log
     if (result != WHIRGPU_OK) return result;
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "autotune");
-    lde_install_plan(log_expansion, best_p);
+    lde_install_plan(log_expansion, best_p, false);
     best->log_n = log_n;
     best->log_expansion = log_expansion;
     best->npass = best_p.npass;
@@ -284,7 +294,7 @@ whirgpu_status whirgpu_ntt_autotune(whirgpu_ctx* c, uint32_t log_n, uint32_t log
     return WHIRGPU_OK;
 }
 
-whirgpu_status whirgpu_ntt_set_plan(const whirgpu_ntt_plan* p) {
+static whirgpu_status install(const whirgpu_ntt_plan* p, bool forced) {
     if (!p) return WHIRGPU_E_INVALID;
     LdePlan q{};
     q.logN = p->log_n;
@@ -296,9 +306,11 @@ whirgpu_status whirgpu_ntt_set_plan(const whirgpu_ntt_plan* p) {
         q.logW[k] = k < (int)p->npass ? p->log_cols[k] : LDE_W_AUTO;
     }
     if (p->npass != 0 && !lde_plan_valid(q)) return WHIRGPU_E_INVALID;
-    lde_install_plan(p->log_expansion, q);
+    lde_install_plan(p->log_expansion, q, forced);
     return WHIRGPU_OK;
 }
+
+whirgpu_status whirgpu_ntt_set_plan(const whirgpu_ntt_plan* p) { return install(p, true); }
 
 whirgpu_status whirgpu_ntt_get_plan(uint32_t log_n, uint32_t log_expansion, whirgpu_ntt_plan* out) {
     if (!out || log_n > TW_LOG) return WHIRGPU_E_INVALID;
@@ -400,7 +412,7 @@ whirgpu_status whirgpu_ntt_load_plans(const char* path, size_t* loaded) {
             pl.log_radix[i] = (uint32_t)r[i];
             pl.log_cols[i] = (uint32_t)w[i];
         }
-        if (whirgpu_ntt_set_plan(&pl) == WHIRGPU_OK) ++n;
+        if (install(&pl, false) == WHIRGPU_OK) ++n;
         p = q;
     }
     if (loaded) *loaded = n;

@@ -60,6 +60,7 @@ struct LdeArgs {
     const u64* tw_hi;
     const u64* tw_lo;
     const struct LdeTables* tables;  // inter-pass factors of the context, or null
+    u32* err;           // device error word (TX_ERR_TIMEOUT), or null
 };
 // Inter-pass twiddle tables of one context.  The pass boundary of a
 // 2^logNs-point (sub-)transform split as 2^logR rows x 2^logS columns
@@ -72,12 +73,13 @@ struct LdeArgs {
 // context; a pass whose table is missing computes its factors by multiplying.
 struct LdeTables {
     static constexpr u32 MAX_LOG = 24;  // largest table: 2^24 words (128 MiB)
-    std::atomic<u64*> tab[(TW_LOG + 1) * (TW_STAGE_LOG + 1)];
+    static constexpr u32 STRIDE = TW_LOG + 1;
+    std::atomic<u64*> tab[(TW_LOG + 1) * STRIDE];  // [logNs * STRIDE + logR]
     LdeTables() {
         for (auto& t : tab) t.store(nullptr);
     }
     const u64* get(u32 logNs, u32 logR) const {
-        return logNs <= TW_LOG && logR <= TW_STAGE_LOG ? tab[logNs * (TW_STAGE_LOG + 1) + logR].load() : nullptr;
+        return logNs <= TW_LOG && logR <= logNs ? tab[logNs * STRIDE + logR].load() : nullptr;
     }
 };
 // The plan launch_lde uses for a 2^logN codeword of a 2^logN / 2^logX message:
@@ -86,7 +88,9 @@ struct LdeTables {
 LdePlan plan_lde(u32 logN, u32 logX);
 LdePlan default_plan_lde(u32 logN);
 bool lde_plan_valid(const LdePlan& p);
-void lde_install_plan(u32 logX, const LdePlan& p);  // p.npass == 0 removes
+// p.npass == 0 removes.  A forced plan's passes are used even where the
+// contraction form (k_dft8.cu) covers the shape.
+void lde_install_plan(u32 logX, const LdePlan& p, bool forced);
 void lde_clear_plans();
 // Incremented by every plan install or clear (captured graphs hold the plans
 // of their capture and are re-captured after a change).
@@ -95,15 +99,23 @@ size_t lde_installed_plans(u32* keys, LdePlan* plans, size_t cap);  // keys: log
 // Launches one LDE with an explicit plan (autotuner).
 int launch_lde_plan(const LdeArgs& a, const LdePlan& pl, cudaStream_t st);
 int launch_lde(const LdeArgs& a, cudaStream_t st);
+// The LDE as two passes of 8-bit contractions (k_dft8.cu): whether the shape is
+// covered, the first pass's output bits (its table in LdeTables is
+// (logN, those bits)), and the launch.
+bool dft8_applicable(u32 logN, u32 logX, u32 planes);
+u32 dft8_first_bits(u32 logN, u32 logX);
+int launch_dft8(const LdeArgs& a, u32 logX, cudaStream_t st);
+int dft8_prepare();
 int lde_prepare();
-// Builds the missing inter-pass tables of `pl` (or of plan_lde(logN, logX))
+// Builds the missing inter-pass tables of `pl` (or of the form launch_lde takes
+// for (logN, logX, planes))
 // whose size fits `room` bytes, on `st`, and waits for them before publishing
 // them.  Returns the bytes allocated, or -1 after a CUDA error (the tables
 // stay missing; the LDE still runs).
 long long lde_tables_prepare_plan(LdeTables& t, const LdePlan& pl, const u64* tw_hi, const u64* tw_lo,
                                   cudaStream_t st, u64 room);
-long long lde_tables_prepare(LdeTables& t, u32 logN, u32 logX, const u64* tw_hi, const u64* tw_lo, cudaStream_t st,
-                             u64 room);
+long long lde_tables_prepare(LdeTables& t, u32 logN, u32 logX, u32 planes, const u64* tw_hi, const u64* tw_lo,
+                             cudaStream_t st, u64 room);
 void lde_tables_free(LdeTables& t);
 // Resident-CTA counts of the sumcheck round kernels on the current device
 // (their grids never leave a partial wave); called once per context.

@@ -229,6 +229,7 @@ int commit_vectors(const Ctx& c, int ci, const uint64_t* const src[3], uint32_t 
     L.tw_hi = c.tw.tw_hi;
     L.tw_lo = c.tw.tw_lo;
     L.tables = c.tw.lde;
+    L.err = &c.tx()->err;
     WG_TIMED(c, FAM_NTT, launch_lde(L, c.st));
     uint32_t* nodes = reinterpret_cast<uint32_t*>(c.ws + cb.nodes);
     WG_TIMED(c, FAM_LEAF, launch_leaves(c.w(cb.planes), cb.N, cb.depth, ncomp, nodes, c.p.params.hash, c.st,

@@ -61,7 +61,7 @@ constexpr unsigned TX_RATE = 168;
 
 // Error bits recorded in TxState::err (never a trap: the host reads them).
 constexpr unsigned TX_ERR_NARG_OVERFLOW = 1u, TX_ERR_HINT_OVERFLOW = 2u, TX_ERR_POW_EXHAUSTED = 4u,
-                   TX_ERR_BAD_INDEX = 8u, TX_ERR_FIELD = 16u;
+                   TX_ERR_BAD_INDEX = 8u, TX_ERR_FIELD = 16u, TX_ERR_TIMEOUT = 32u;
 
 struct TxState {
     u64 hasher[25];
