@@ -827,8 +827,8 @@ int launch_lde_plan(const LdeArgs& L, const LdePlan& pl, cudaStream_t st) {
 // The two contraction passes have a floor of 19-30 us (their constants and one
 // tile's round trip); below 2^20 words the butterfly passes take 9-25 us.
 // Measured (us, contraction / butterfly): 48 planes 2^12 -> 2^14 31 / 25,
-// 16 planes 2^14 -> 2^16 29 / 33, 16 planes 2^20 -> 2^22 923 / 1658, 48 planes
-// 2^16 -> 2^21 1157 / 1846, 48 planes 2^12 -> 2^20 435 / 752.
+// 16 planes 2^14 -> 2^16 29 / 33, 16 planes 2^20 -> 2^22 682 / 1658, 48 planes
+// 2^16 -> 2^21 853 / 1846, 48 planes 2^12 -> 2^20 338 / 752.
 static bool use_dft8(u32 logN, u32 logX, u32 planes) {
     if (((u64)planes << logN) < (1ull << 20) || !dft8_applicable(logN, logX, planes)) return false;
     std::lock_guard<std::mutex> lk(g_plan_mu);
@@ -839,8 +839,11 @@ int launch_lde(const LdeArgs& L, cudaStream_t st) {
     u32 lm = 0;
     while ((1ull << lm) < L.m) ++lm;
     const u32 logX = L.logN > lm ? L.logN - lm : 0;
+    // The contraction passes load 16-byte word pairs of the message and the scratch.
+    auto al16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     if (L.logN == lm + logX && L.m == 1ull << lm && L.tables && use_dft8(L.logN, logX, L.planes) &&
-        L.tables->get(L.logN, dft8_first_bits(L.logN, logX)))
+        L.tables->get(L.logN, dft8_first_bits(L.logN, logX)) && al16(L.src[0]) && al16(L.src[1]) && al16(L.src[2]) &&
+        al16(L.tmp))
         return launch_dft8(L, logX, st);
     return launch_lde_plan(L, plan_lde(L.logN, logX), st);
 }
