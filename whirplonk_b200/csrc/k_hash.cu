@@ -35,10 +35,10 @@ __device__ __forceinline__ void load_node(const u32* nodes, u64 idx, unsigned* m
 
 // The engine a configuration's hash_id selects (irs_commit.hpp:62-74).
 constexpr int HASH_BLAKE3 = 0, HASH_SHA256 = 1;
-template <int H>
+template <int H, bool FMA = true>
 __device__ __forceinline__ void hash64(const unsigned m[16], unsigned out[8]) {
-    if (H == HASH_SHA256) sha256_hash64(m, out);
-    else b3_hash64(m, out);
+    if (H == HASH_SHA256) sha256_hash64<FMA>(m, out);
+    else b3_hash64<FMA>(m, out);
 }
 
 // Row i = words w = 0 .. depth*ncomp-1 with w -> (element w / ncomp, component w % ncomp),
@@ -268,14 +268,16 @@ int launch_leaves(const u64* planes, u64 N, u32 depth, u32 ncomp, u32* nodes, in
 // `blk`, whose 2^levels children sit at level level_in from node blk 2^levels
 // on; every produced level is written to global memory and the working level
 // kept in shared memory.  CG: the children were written by other CTAs of the
-// same launch, so they are read through L2.  Ends with a CTA barrier.
+// same launch, so they are read through L2.  FMA: see blake3.cuh (a lone
+// subtree is a chain of hashes, many at once fill the pipes).  Ends with a CTA
+// barrier.
 __device__ __forceinline__ void load_node_cg(const u32* nodes, u64 idx, unsigned* m) {
     const uint4* p = reinterpret_cast<const uint4*>(nodes + idx * 8);
     const uint4 a = __ldcg(p), b = __ldcg(p + 1);
     m[0] = a.x; m[1] = a.y; m[2] = a.z; m[3] = a.w;
     m[4] = b.x; m[5] = b.y; m[6] = b.z; m[7] = b.w;
 }
-template <int H, bool CG>
+template <int H, bool CG, bool FMA>
 __device__ __forceinline__ void merkle_subtree(u32* nodes, u32 logN, u32 level_in, u32 levels, u64 blk,
                                                unsigned (*buf)[256 * 8]) {
     const u32 nparents = 1u << (levels - 1);
@@ -292,7 +294,7 @@ __device__ __forceinline__ void merkle_subtree(u32* nodes, u32 logN, u32 level_i
             load_node(nodes, in_off + child + 1, m + 8);
         }
         unsigned cv[8];
-        hash64<H>(m, cv);
+        hash64<H, FMA>(m, cv);
         store_node(nodes, out_off + (blk << (levels - 1)) + t, cv);
 #pragma unroll
         for (int k = 0; k < 8; ++k) buf[0][t * 8 + k] = cv[k];
@@ -307,7 +309,7 @@ __device__ __forceinline__ void merkle_subtree(u32* nodes, u32 logN, u32 level_i
 #pragma unroll
             for (int k = 0; k < 16; ++k) m[k] = buf[cur][t * 16 + k];
             unsigned cv[8];
-            hash64<H>(m, cv);
+            hash64<H, FMA>(m, cv);
             store_node(nodes, off + (blk << (levels - 1 - lv)) + t, cv);
 #pragma unroll
             for (int k = 0; k < 8; ++k) buf[cur ^ 1][t * 8 + k] = cv[k];
@@ -337,13 +339,13 @@ __device__ __forceinline__ void merkle_send_root(const u32* nodes, u32 logN, TxS
 
 // One CTA hashes a subtree of height `levels` whose children sit at level
 // `level_in`; every produced level is written to global memory.
-template <int H>
+template <int H, bool FMA>
 __global__ void __launch_bounds__(256) k_merkle(u32* nodes, u32 logN, u32 level_in, u32 levels, TxState* tx,
                                                 ProofScalars* sc, int commit_idx, int n_ood, int finish,
                                                 u64 node_stride) {
     __shared__ unsigned buf[2][256 * 8];
     nodes += blockIdx.y * node_stride;
-    if (levels > 0) merkle_subtree<H, false>(nodes, logN, level_in, levels, blockIdx.x, buf);
+    if (levels > 0) merkle_subtree<H, false, FMA>(nodes, logN, level_in, levels, blockIdx.x, buf);
     if (finish && tx && threadIdx.x < 32) merkle_send_root(nodes, logN, tx, sc, commit_idx, n_ood);
 }
 
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(256) k_merkle_tail(u32* nodes, u32 logN, u32 l
                                                      ProofScalars* sc, int commit_idx, int n_ood) {
     __shared__ unsigned buf[2][256 * 8];
     __shared__ bool last;
-    merkle_subtree<H, false>(nodes, logN, level_in, 9, blockIdx.x, buf);
+    merkle_subtree<H, false, false>(nodes, logN, level_in, 9, blockIdx.x, buf);
     if (threadIdx.x == 0) {
         __threadfence();  // this CTA's subtree root (written by thread 0) before its ticket
         last = atomicAdd(&sc->counters[CTR_MERKLE_TAIL], 1u) == gridDim.x - 1;
@@ -365,7 +367,7 @@ __global__ void __launch_bounds__(256) k_merkle_tail(u32* nodes, u32 logN, u32 l
     __syncthreads();
     if (!last) return;
     __threadfence();
-    merkle_subtree<H, true>(nodes, logN, level_in + 9, logN - level_in - 9, 0, buf);
+    merkle_subtree<H, true, false>(nodes, logN, level_in + 9, logN - level_in - 9, 0, buf);
     if (threadIdx.x < 32) merkle_send_root(nodes, logN, tx, sc, commit_idx, n_ood);
     if (threadIdx.x == 0) sc->counters[CTR_MERKLE_TAIL] = 0;
 }
@@ -417,7 +419,7 @@ static int merkle_levels_h(u32* nodes, u32 logN, TxState* tx, ProofScalars* sc, 
     }
     if (logN == 0) {
         if (tx) {
-            k_merkle<H><<<dim3(1, count), 32, 0, st>>>(nodes, logN, 0, 0, tx, sc, commit_idx, n_ood, 1, node_stride);
+            k_merkle<H, false><<<dim3(1, count), 32, 0, st>>>(nodes, logN, 0, 0, tx, sc, commit_idx, n_ood, 1, node_stride);
             count_launches(1);
         }
         return 0;
@@ -431,8 +433,11 @@ static int merkle_levels_h(u32* nodes, u32 logN, TxState* tx, ProofScalars* sc, 
         const u32 levels = (logN - level) < 9 ? (logN - level) : 9;
         const u32 ctas = 1u << (logN - level - levels);
         const int finish = (level + levels == logN) ? 1 : 0;
-        k_merkle<H><<<dim3(ctas, count), 256, 0, st>>>(nodes, logN, level, levels, tx, sc, commit_idx, n_ood, finish,
-                                                    node_stride);
+        // From four CTAs a SM on the hashes of the wide levels fill the ALU pipe:
+        // 64 trees of 2^13 leaves take 189 us end to end this way, 199 us with
+        // the short chains.
+        auto* const k = (u64)ctas * count >= 4ull * device_sms() ? k_merkle<H, true> : k_merkle<H, false>;
+        k<<<dim3(ctas, count), 256, 0, st>>>(nodes, logN, level, levels, tx, sc, commit_idx, n_ood, finish, node_stride);
         count_launches(1);
         level += levels;
     }
