@@ -3,6 +3,8 @@
 // work grinding, in-domain openings (indices, row hints, Merkle paths) and
 // the final-vector message.  Protocol order and byte layout follow
 // cpp/include/whir/protocols/whir/whir_prover.hpp:56-407.
+#include <algorithm>
+
 #include "launch.h"
 #include "blake3.cuh"
 #include "sha256.cuh"
@@ -178,11 +180,15 @@ __global__ void k_pow_finish(TxState* tx, ProofScalars* sc, int slot) {
     wtx_store(t, tx);
 }
 
-int launch_pow(TxState* tx, ProofScalars* sc, u64 threshold, int slot, int hash, cudaStream_t st) {
+int launch_pow_search(TxState* tx, ProofScalars* sc, u64 threshold, int hash, cudaStream_t st) {
     if (threshold == ~0ull) return 0;  // zero difficulty: nothing sent (proof_of_work.hpp:241)
     k_pow_challenge<<<1, 32, 0, st>>>(tx, sc);
     count_launches(1);
-    launch_pow_grind_only(sc, threshold, hash, st);
+    return launch_pow_grind_only(sc, threshold, hash, st);
+}
+int launch_pow(TxState* tx, ProofScalars* sc, u64 threshold, int slot, int hash, cudaStream_t st) {
+    if (threshold == ~0ull) return 0;
+    launch_pow_search(tx, sc, threshold, hash, st);
     k_pow_finish<<<1, 32, 0, st>>>(tx, sc, slot);
     count_launches(1);
     return 0;
@@ -228,8 +234,8 @@ int launch_squeeze_challenges(TxState* tx, ProofScalars* sc, int slot, int count
 
 // ---------------------------------------------------------------------------
 // Opening (irs_commit.hpp:600-713, challenge_indices.hpp:56-119,
-// merkle_tree.hpp:165-211) of nwit commitments at the same rows, one CTA of
-// 1024 threads:
+// merkle_tree.hpp:165-211) of nwit commitments at the same rows:
+//   0. (after a PoW search) the nonce message (proof_of_work.hpp);
 //   1. squeeze q * ceil(log2(N)/8) bytes, index = big-endian bytes mod N;
 //   2. per commitment: hint u64 (q * depth), the q rows in index order
 //      (duplicates kept), then its Merkle hints -- sorted, deduplicated
@@ -238,216 +244,245 @@ int launch_squeeze_challenges(TxState* tx, ProofScalars* sc, int slot, int count
 //      and indices, so its hint block has the same length;
 //   3. (STIR) point gen^idx and value <rows, vector_rlc (x) eq_weights(last
 //      folding randomness)> over the rows of all commitments side by side
-//      (whir_prover.hpp:283-310).
+//      (whir_prover.hpp:283-310);
+//   4. (STIR) the combination over the new commitment's OOD points/values and
+//      these: RLC = geometric_challenge(O + q), sum += <rlc, values>
+//      (whir_prover.hpp:310-336).
+//
+// A chain of dependent loads and transcript steps, so latency is all that
+// counts.  Warp 0 of a CTA runs the transcript -- nonce, index bytes, then the
+// RLC challenge and its powers, which wait for no value -- while the other
+// warps sort the indices and gather rows, values and hashes.  Up to OPEN_CTAS
+// CTAs do the transcript and the sort each for itself (the same bytes; no CTA
+// waits for another) and share the gathering; the last one to finish (a
+// self-resetting ticket) sums the combination and stores the transcript.
+// Against one CTA of 1024 threads between a nonce launch and a combination
+// launch (B200, a whole proof): n = 16 rate 1/4 823 -> 766 us, n = 18 rate 1/2
+// 1007 -> 935 us.  The same split with the powers after the values gained 20 us
+// less.
 // ---------------------------------------------------------------------------
-constexpr int OPEN_THREADS = 1024;
+constexpr int OPEN_THREADS = 512, OPEN_WARPS = OPEN_THREADS / 32;
+constexpr int OPEN_GATHER = OPEN_THREADS - 32;  // threads of the gathering warps
+constexpr u32 OPEN_CTAS = 8, OPEN_MAX_LOGN = 26;
 
-// Exclusive prefix count of `flag` over the CTA; *total receives the sum.
-__device__ u32 block_scan(bool flag, u32* warp_tot, u32* total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const unsigned bal = __ballot_sync(0xFFFFFFFFu, flag);
-    const u32 pre = __popc(bal & ((1u << lane) - 1));
-    if (lane == 0) warp_tot[warp] = __popc(bal);
-    __syncthreads();
-    if (warp == 0) {
-        u32 v = lane < (int)(blockDim.x >> 5) ? warp_tot[lane] : 0;
-        u32 incl = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            u32 t = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += t;
-        }
-        warp_tot[lane] = incl - v;  // exclusive
-        if (lane == 31) *total = incl;
-    }
-    __syncthreads();
-    const u32 r = warp_tot[warp] + pre;
-    __syncthreads();
+// Barrier of the gathering warps, and the same counting `v`.
+__device__ __forceinline__ void gather_sync() { asm volatile("bar.sync 1, %0;" ::"n"(OPEN_GATHER) : "memory"); }
+__device__ __forceinline__ u32 gather_count(bool v) {
+    u32 r;
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.popc.u32 %0, 1, %2, p;\n\t}"
+                 : "=r"(r)
+                 : "r"((u32)v), "n"(OPEN_GATHER)
+                 : "memory");
     return r;
 }
 
 __global__ void __launch_bounds__(OPEN_THREADS) k_open(OpenArgs a) {
     __shared__ u64 idx_s[MAX_QUERIES];
     __shared__ u64 cur[MAX_QUERIES];
-    __shared__ u32 warp_tot[32];
-    __shared__ u32 total;
+    __shared__ unsigned char dup[MAX_QUERIES];
     __shared__ E3 eqw[MAX_DEPTH];
-    __shared__ u64 hint_base;
-    __shared__ unsigned char idx_bytes[MAX_QUERIES * 8];
-    __shared__ unsigned char occ[MAX_QUERIES];
-    __shared__ u32 lvl_cnt[32];
-    const TxState* tx = a.tx;  // hint pointers and capacity only; warp 0 carries the sponge
+    __shared__ unsigned char idx_bytes[MAX_QUERIES * 4];
+    __shared__ u32 cnt[OPEN_MAX_LOGN][MAX_QUERIES / 32];  // emitted siblings per level and chunk of 32 nodes, then their prefix
+    __shared__ u32 lvl[OPEN_MAX_LOGN + 1];                // siblings of the levels below, and of all
+    __shared__ E3 red[OPEN_WARPS];
+    __shared__ bool last;
+    const TxState* tx = a.tx;  // the hint stream (unchanged until the last CTA's store)
     ProofScalars* sc = a.sc;
-    const u32 t = threadIdx.x;
+    const u32 t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const u32 q = a.q;
     const u32 nbytes = (a.logN + 7) / 8;
     const u32 nwit = a.nwit;
     const bool x2 = tx->deg == 2;  // GoldilocksExt2 target field
+    const u64 hint_base = tx->hints_len;
+    const int count = a.ood_offset + (int)q;  // values of the STIR combination
 
-    // 1. indices: warp 0 squeezes q * nbytes bytes (big-endian per index)
     WarpTx wt;
-    if (t < 32) {
+    if (warp == 0) {
         wtx_load(wt, a.tx);
+        if (a.pow_slot >= 0) {
+            const u64 n = sc->pow_best;
+            if (n == ~0ull) wt.err |= TX_ERR_POW_EXHAUSTED;
+            if (blockIdx.x == 0 && lane == 0 && a.pow_slot < MAX_COMMITS + 4) sc->pow_nonces[a.pow_slot] = n;
+            wtx_message_u64(wt, n);
+        }
         if (a.N != 1) wtx_squeeze_bytes(wt, idx_bytes, q * nbytes);
-    }
-    __syncthreads();
-    for (u32 i = t; i < q; i += blockDim.x) {
-        u64 acc = 0;
-        for (u32 k = 0; k < nbytes; ++k) acc = (acc << 8) | idx_bytes[i * nbytes + k];
-        idx_s[i] = a.N == 1 ? 0 : (acc & (a.N - 1));  // N is a power of two
-    }
-    if (t == 0) hint_base = wt.hints_len;
-    // eq weights of the last `fold` folding challenges (multilinear_point.hpp:40-62),
-    // one entry per thread of warps 1.. (they do not wait for warp 0's squeeze)
-    if (a.stir && t >= 32 && t - 32 < (1u << a.fold)) {
-        const u32 i = t - 32;
-        E3 acc = e3_one();
-        for (u32 k = 0; k < a.fold; ++k) {
-            const E3 r = sc->sc_r[a.r_offset + k];
-            const bool bit = (i >> (a.fold - 1 - k)) & 1;
-            acc = ef_mul(acc, bit ? r : e3_sub(e3_one(), r), x2);
-        }
-        eqw[i] = acc;
-    }
-    for (u32 s2 = t; s2 < (u32)MAX_QUERIES; s2 += blockDim.x) occ[s2] = 0;
-    __syncthreads();
-    for (u32 i = t; i < q; i += blockDim.x) sc->indices[i] = idx_s[i];
-
-    // Sort + dedup: a first occurrence v goes to slot #{j : idx_j < v}; distinct
-    // values get distinct, order-preserving slots, compacted with a CTA scan.
-    if (t < q) {
-        const u64 v = idx_s[t];
-        u32 lt = 0;
-        bool dup = false;
-        for (u32 j = 0; j < q; ++j) {
-            const u64 o = idx_s[j];
-            lt += (o < v) ? 1u : 0u;
-            dup |= (o == v && j < t);
-        }
-        if (!dup) { cur[lt] = v; occ[lt] = 1; }
-    }
-    __syncthreads();
-    const bool present = t < q && occ[t];
-    const u64 pv = present ? cur[t] : 0;
-    const u32 pos = block_scan(present, warp_tot, &total);
-    const u32 u = total;
-    if (present) cur[pos] = pv;
-    __syncthreads();
-
-    // Merkle levels.  Per level L the nodes are the distinct values of
-    // cur[j] >> L (cur is sorted, so equal values are adjacent); a node x emits
-    // its sibling x ^ 1 unless the sibling is itself a node.  Warp L handles
-    // level L: it walks cur in chunks of 32 lanes and ranks its emitters with a
-    // ballot.  The per-level counts are prefix-summed, so every warp writes its
-    // siblings at the reference's position (level by level, increasing x within
-    // a level).
-    const u32 warp = t >> 5, lane = t & 31;
-    auto present_at = [&](u64 y, u32 L) -> bool {  // is y a node of level L?
-        u32 lo = 0, hi = u;
-        while (lo < hi) {
-            const u32 mid = (lo + hi) >> 1;
-            if ((cur[mid] >> L) < y) lo = mid + 1;
-            else hi = mid;
-        }
-        return lo < u && (cur[lo] >> L) == y;
-    };
-    auto emits = [&](u32 j, u32 L) -> bool {
-        if (j >= u) return false;
-        const u64 x = cur[j] >> L;
-        const bool first = j == 0 || (cur[j - 1] >> L) != x;
-        return first && !present_at(x ^ 1, L);
-    };
-    if (warp < a.logN) {
-        u32 cnt = 0;
-        for (u32 j0 = 0; j0 < u; j0 += 32) cnt += __popc(__ballot_sync(0xFFFFFFFFu, emits(j0 + lane, warp)));
-        if (lane == 0) lvl_cnt[warp] = cnt;
-    }
-    __syncthreads();
-    u64 merkle_bytes = 0;
-    for (u32 k = 0; k < a.logN; ++k) merkle_bytes += 32ull * lvl_cnt[k];
-    const u64 esz = 8ull * a.ncomp;
-    const u64 row_bytes = esz * a.depth;
-    const u64 row_hint = 8 + row_bytes * q;
-    const u64 blk = row_hint + merkle_bytes;  // hint bytes of one commitment
-    const bool fits = hint_base + blk * nwit <= tx->hints_cap;
-
-    // 2a. row hints.  Every hint word sits at a multiple of 8 bytes from the
-    // commitment's hint block, so when the block starts 8-byte aligned (the
-    // hints stream holds whole words) a word is one 8-byte store.
-    const bool hints_al8 = (reinterpret_cast<uintptr_t>(tx->hints + hint_base) & 7) == 0;
-    if (fits) {
-        const u32 rw = a.depth * a.ncomp;  // words per row (<= MAX_DEPTH * 3)
-        const u32 nwords = q * rw;
-        for (u32 w = 0; w < nwit; ++w) {
-            unsigned char* hb = tx->hints + hint_base + w * blk;
-            const u64* planes = a.planes + w * a.planes_stride;
-            if (t == 0) {
-                const u64 len = (u64)q * a.depth;
-                for (int k = 0; k < 8; ++k) hb[k] = (unsigned char)(len >> (8 * k));
+    } else if (a.stir) {
+        // eq weights of the last `fold` folding challenges (multilinear_point.hpp:40-62)
+        for (u32 i = t - 32; i < (1u << a.fold); i += OPEN_GATHER) {
+            E3 acc = e3_one();
+            for (u32 k = 0; k < a.fold; ++k) {
+                const E3 r = sc->sc_r[a.r_offset + k];
+                const bool bit = (i >> (a.fold - 1 - k)) & 1;
+                acc = ef_mul(acc, bit ? r : e3_sub(e3_one(), r), x2);
             }
-            for (u32 x = t; x < nwords; x += blockDim.x) {
-                const u32 qi = x / rw, rem = x - qi * rw;
-                const u32 el = rem / a.ncomp, c = rem - el * a.ncomp;
-                const u64 v = planes[((u64)c * a.depth + el) * a.N + codeword_row(idx_s[qi], a.logN, a.perm_log_e)];
-                unsigned char* dst = hb + 8 + qi * row_bytes + (u64)el * esz + 8ull * c;
-                if (hints_al8) {
-                    *reinterpret_cast<u64*>(dst) = v;
-                } else {
-#pragma unroll 1
-                    for (int k = 0; k < 8; ++k) dst[k] = (unsigned char)(v >> (8 * k));
+            eqw[i] = acc;
+        }
+    }
+    __syncthreads();
+    u64 blk = 0;  // hint bytes of one commitment (gathering warps)
+    bool fits = true;
+    if (warp == 0) {
+        // Every CTA writes the same powers to the same place.
+        if (a.stir) wtx_geometric(wt, sc->stir_rlc, count);
+    } else {
+        const u32 g = t - 32;  // gathering thread
+        const u32 ggw = blockIdx.x * (OPEN_WARPS - 1) + warp - 1, ggws = gridDim.x * (OPEN_WARPS - 1);
+        for (u32 i = g; i < q; i += OPEN_GATHER) {
+            u64 acc = 0;
+            for (u32 k = 0; k < nbytes; ++k) acc = (acc << 8) | idx_bytes[i * nbytes + k];
+            acc = a.N == 1 ? 0 : (acc & (a.N - 1));  // N is a power of two
+            idx_s[i] = acc;
+            if (blockIdx.x == 0) sc->indices[i] = acc;
+        }
+        gather_sync();
+
+        // 3. STIR point and value of each opened row: a warp per row, its lanes
+        //    over the row's elements (all commitments side by side), a warp sum.
+        if (a.stir) {
+            const u32 dmask = (1u << a.fold) - 1;
+            const u32 elems = nwit * a.depth;
+            for (u32 i = ggw; i < q; i += ggws) {
+                const u64 id = codeword_row(idx_s[i], a.logN, a.perm_log_e);  // natural row = exponent of its point
+                E3 val = e3_zero();
+                for (u32 k = lane; k < elems; k += 32) {
+                    const u32 w = k / a.depth, el = k - w * a.depth;
+                    const u64* planes = a.planes + w * a.planes_stride;
+                    E3 term;
+                    if (a.ncomp == 1) {
+                        term = e3_mul_base(eqw[el & dmask], planes[(u64)el * a.N + id]);
+                    } else if (a.ncomp == 2) {  // Ext2 rows: planes c0, c1
+                        term = ef_mul(E3{planes[(u64)el * a.N + id], planes[((u64)a.depth + el) * a.N + id], 0},
+                                      eqw[el & dmask], true);
+                    } else {
+                        term = e3_mul(E3{planes[(u64)el * a.N + id], planes[((u64)a.depth + el) * a.N + id],
+                                         planes[((u64)2 * a.depth + el) * a.N + id]},
+                                      eqw[el & dmask]);
+                    }
+                    if (a.use_vrlc) term = ef_mul(term, sc->vrlc[w * (a.depth >> a.fold) + (el >> a.fold)], x2);
+                    val = e3_add(val, term);
+                }
+                val = e3_warp_sum(val);
+                if (lane == 0) {
+                    sc->stir_pts[a.ood_offset + i] = e3_base(gl_pow(a.gen, id));
+                    sc->stir_vals[a.ood_offset + i] = val;
                 }
             }
         }
-    }
 
-    // 3. STIR point and value of each opened row: a warp per row, its lanes over
-    //    the row's elements (all commitments side by side), a warp sum at the end.
-    if (a.stir) {
-        const u32 dmask = (1u << a.fold) - 1;
-        const u32 total = nwit * a.depth;
-        const u32 nwarps = blockDim.x >> 5;
-        for (u32 i = warp; i < q; i += nwarps) {
-            const u64 id = codeword_row(idx_s[i], a.logN, a.perm_log_e);  // natural row = exponent of its point
-            E3 val = e3_zero();
-            for (u32 k = lane; k < total; k += 32) {
-                const u32 w = k / a.depth, el = k - w * a.depth;
+        // Sort + dedup: a value goes to slot #{distinct values below it}.  Two
+        // lanes share an index's comparisons.
+        u32 u = 0;
+        for (u32 i0 = 0; i0 < q; i0 += OPEN_GATHER / 2) {
+            const u32 i = i0 + (g >> 1);
+            const u64 v = i < q ? idx_s[i] : 0;
+            bool d = false;
+            for (u32 j = g & 1; j < i && i < q; j += 2) d |= idx_s[j] == v;
+            d |= __shfl_xor_sync(0xFFFFFFFFu, (int)d, 1);
+            if (i < q) dup[i] = d;
+            u += gather_count(i < q && !d && (g & 1) == 0);
+        }
+        for (u32 i0 = 0; i0 < q; i0 += OPEN_GATHER / 2) {
+            const u32 i = i0 + (g >> 1);
+            const u64 v = i < q ? idx_s[i] : 0;
+            u32 lt = 0;
+            for (u32 j = g & 1; j < q; j += 2) lt += idx_s[j] < v && !dup[j];
+            lt += __shfl_xor_sync(0xFFFFFFFFu, lt, 1);
+            if (i < q && !dup[i] && (g & 1) == 0) cur[lt] = v;
+        }
+        gather_sync();
+
+        // Merkle levels.  Per level L the nodes are the distinct values x of
+        // cur[j] >> L (cur is sorted, so equal values are adjacent); x emits its
+        // sibling x ^ 1 unless the sibling is itself a node, i.e. the
+        // neighbouring distinct value: an odd x decides at its first j, an even
+        // x at its last.  Siblings are emitted level by level, increasing x
+        // within a level.
+        const u32 nchunk = (u + 31) / 32;
+        auto emits = [&](u32 j, u32 L) -> bool {
+            if (j >= u) return false;
+            const u64 x = cur[j] >> L;
+            if (x & 1) {
+                if (j == 0) return true;
+                const u64 p = cur[j - 1] >> L;
+                return p != x && p != x - 1;
+            }
+            if (j + 1 == u) return true;
+            const u64 n = cur[j + 1] >> L;
+            return n != x && n != x + 1;
+        };
+        for (u32 it = warp - 1; it < a.logN * nchunk; it += OPEN_WARPS - 1) {
+            const u32 L = it / nchunk, c = it % nchunk;
+            const u32 m = __popc(__ballot_sync(0xFFFFFFFFu, emits(c * 32 + lane, L)));
+            if (lane == 0) cnt[L][c] = m;
+        }
+        gather_sync();
+        auto exclusive = [&](u32 v, u32& total) {
+            u32 incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const u32 w = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= (u32)o) incl += w;
+            }
+            total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            return incl - v;
+        };
+        for (u32 L = warp - 1; L < a.logN; L += OPEN_WARPS - 1) {
+            u32 total;
+            const u32 e = exclusive(lane < nchunk ? cnt[L][lane] : 0, total);
+            if (lane < nchunk) cnt[L][lane] = e;
+            if (lane == 0) lvl[L] = total;
+        }
+        gather_sync();
+        if (warp == 1) {
+            u32 total;
+            const u32 e = exclusive(lane < a.logN ? lvl[lane] : 0, total);
+            if (lane <= a.logN) lvl[lane] = e;
+        }
+        gather_sync();
+        const u64 merkle_bytes = 32ull * lvl[a.logN];
+        const u64 esz = 8ull * a.ncomp;
+        const u64 row_bytes = esz * a.depth;
+        const u64 row_hint = 8 + row_bytes * q;
+        blk = row_hint + merkle_bytes;
+        fits = hint_base + blk * nwit <= tx->hints_cap;
+
+        // 2a. row hints.  Every hint word sits at a multiple of 8 bytes from the
+        // commitment's hint block, so when the block starts 8-byte aligned (the
+        // hints stream holds whole words) a word is one 8-byte store.
+        const bool hints_al8 = (reinterpret_cast<uintptr_t>(tx->hints + hint_base) & 7) == 0;
+        if (fits) {
+            const u32 rw = a.depth * a.ncomp;  // words per row (<= MAX_DEPTH * 3)
+            const u32 nwords = q * rw;
+            for (u32 w = 0; w < nwit; ++w) {
+                unsigned char* hb = tx->hints + hint_base + w * blk;
                 const u64* planes = a.planes + w * a.planes_stride;
-                E3 term;
-                if (a.ncomp == 1) {
-                    term = e3_mul_base(eqw[el & dmask], planes[(u64)el * a.N + id]);
-                } else if (a.ncomp == 2) {  // Ext2 rows: planes c0, c1
-                    term = ef_mul(E3{planes[(u64)el * a.N + id], planes[((u64)a.depth + el) * a.N + id], 0},
-                                  eqw[el & dmask], true);
-                } else {
-                    term = e3_mul(E3{planes[(u64)el * a.N + id], planes[((u64)a.depth + el) * a.N + id],
-                                     planes[((u64)2 * a.depth + el) * a.N + id]},
-                                  eqw[el & dmask]);
+                if (g == 0 && blockIdx.x == 0) {
+                    const u64 len = (u64)q * a.depth;
+                    for (int k = 0; k < 8; ++k) hb[k] = (unsigned char)(len >> (8 * k));
                 }
-                if (a.use_vrlc) term = ef_mul(term, sc->vrlc[w * (a.depth >> a.fold) + (el >> a.fold)], x2);
-                val = e3_add(val, term);
+                for (u32 x = blockIdx.x * OPEN_GATHER + g; x < nwords; x += gridDim.x * OPEN_GATHER) {
+                    const u32 qi = x / rw, rem = x - qi * rw;
+                    const u32 el = rem / a.ncomp, c = rem - el * a.ncomp;
+                    const u64 v = planes[((u64)c * a.depth + el) * a.N + codeword_row(idx_s[qi], a.logN, a.perm_log_e)];
+                    unsigned char* dst = hb + 8 + qi * row_bytes + (u64)el * esz + 8ull * c;
+                    if (hints_al8) {
+                        *reinterpret_cast<u64*>(dst) = v;
+                    } else {
+#pragma unroll 1
+                        for (int k = 0; k < 8; ++k) dst[k] = (unsigned char)(v >> (8 * k));
+                    }
+                }
             }
-            val = e3_warp_sum(val);
-            if (lane == 0) {
-                sc->stir_pts[a.ood_offset + i] = e3_base(gl_pow(a.gen, id));
-                sc->stir_vals[a.ood_offset + i] = val;
-            }
-        }
-    }
-
-    // 2b. Merkle hints of every commitment
-    if (warp < a.logN) {
-        const u32 L = warp;
-        u64 lvl_base = row_hint;
-        for (u32 k = 0; k < L; ++k) lvl_base += 32ull * lvl_cnt[k];
-        const u64 level_off = (2ull << a.logN) - (2ull << (a.logN - L));
-        u32 rank = 0;
-        for (u32 j0 = 0; j0 < u; j0 += 32) {
-            const u32 j = j0 + lane;
-            const bool e = emits(j, L);
-            const unsigned m = __ballot_sync(0xFFFFFFFFu, e);
-            if (e && fits) {
+            // 2b. Merkle hints of every commitment: a warp per level and chunk.
+            for (u32 it = ggw; it < a.logN * nchunk; it += ggws) {
+                const u32 L = it / nchunk, c = it % nchunk;
+                const u32 j = c * 32 + lane;
+                const bool e = emits(j, L);
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, e);
+                if (!e) continue;
+                const u64 level_off = (2ull << a.logN) - (2ull << (a.logN - L));
                 const u64 x = cur[j] >> L;
-                const u64 rel = lvl_base + 32ull * (rank + __popc(m & ((1u << lane) - 1)));
+                const u64 rel = row_hint + 32ull * (lvl[L] + cnt[L][c] + __popc(m & ((1u << lane) - 1)));
                 for (u32 w = 0; w < nwit; ++w) {
                     const u32* nodes = a.nodes + w * a.nodes_stride;
                     const uint4* src = reinterpret_cast<const uint4*>(nodes + (level_off + (x ^ 1)) * 8);
@@ -466,50 +501,55 @@ __global__ void __launch_bounds__(OPEN_THREADS) k_open(OpenArgs a) {
                     }
                 }
             }
-            rank += __popc(m);
         }
     }
-    if (t < 32) {
-        if (!fits) wt.err |= TX_ERR_HINT_OVERFLOW;
-        else wt.hints_len = hint_base + blk * nwit;
+
+    // The last CTA: every CTA has read the transcript and written its values.
+    __threadfence();
+    __syncthreads();
+    if (t == 32) {
+        last = atomicAdd(&sc->counters[CTR_OPEN], 1u) == gridDim.x - 1;
+        cur[0] = blk;  // to warp 0
+        cur[1] = fits;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (a.stir) {
+        if (t < (u32)a.ood_offset) {
+            sc->stir_pts[t] = sc->ood_pts[a.rlc_commit][t];
+            sc->stir_vals[t] = sc->ood_vals[a.rlc_commit][t];
+        }
+        E3 acc = e3_zero();
+        for (int j = t; j < count; j += OPEN_THREADS) {
+            const E3* v = j < a.ood_offset ? &sc->ood_vals[a.rlc_commit][j] : &sc->stir_vals[j];
+            const E3* r = &sc->stir_rlc[j];
+            acc = e3_add(acc, ef_mul(E3{__ldcg(&r->c0), __ldcg(&r->c1), __ldcg(&r->c2)},
+                                     E3{__ldcg(&v->c0), __ldcg(&v->c1), __ldcg(&v->c2)}, x2));
+        }
+        acc = e3_warp_sum(acc);
+        if (lane == 0) red[warp] = acc;
+        __syncthreads();
+        if (warp == 0) {
+            acc = e3_warp_sum(lane < OPEN_WARPS ? red[lane] : e3_zero());
+            if (lane == 0) sc->sum = e3_add(sc->sum, acc);
+        }
+    }
+    if (warp == 0) {
+        if (!cur[1]) wt.err |= TX_ERR_HINT_OVERFLOW;
+        else wt.hints_len = hint_base + cur[0] * nwit;
         wtx_store(wt, a.tx);
+        if (lane == 0) sc->counters[CTR_OPEN] = 0;
     }
 }
 
 int launch_open(const OpenArgs& a, cudaStream_t st) {
     if (a.q > (u32)MAX_QUERIES || (1u << a.fold) > (u32)MAX_DEPTH || a.nwit < 1 || a.nwit > (u32)MAX_WITNESSES) return -1;
     if (a.stir && (a.depth & ((1u << a.fold) - 1)) != 0) return -1;
-    k_open<<<1, OPEN_THREADS, 0, st>>>(a);
-    count_launches(1);
-    return 0;
-}
-
-// STIR combination: the new commitment's OOD points/values first, then the
-// in-domain ones written by k_open; RLC = geometric_challenge(O + q);
-// sum += <rlc, values>.
-// One warp.
-__global__ void k_stir_rlc(TxState* tx, ProofScalars* sc, int commit_idx, int n_ood, int q) {
-    if (threadIdx.x >= 32) return;
-    const int l = threadIdx.x;
-    if (l < n_ood) {
-        sc->stir_pts[l] = sc->ood_pts[commit_idx][l];
-        sc->stir_vals[l] = sc->ood_vals[commit_idx][l];
-    }
-    __syncwarp();
-    const int count = n_ood + q;
-    WarpTx t;
-    wtx_load(t, tx);
-    wtx_geometric(t, sc->stir_rlc, count);
-    wtx_store(t, tx);
-    E3 acc = e3_zero();
-    for (int j = l; j < count; j += 32) acc = e3_add(acc, ef_mul(sc->stir_rlc[j], sc->stir_vals[j], t.deg == 2));
-    acc = wtx_sum(acc);
-    if (l == 0) sc->sum = e3_add(sc->sum, acc);
-}
-
-int launch_stir_rlc(TxState* tx, ProofScalars* sc, int commit_idx, int n_ood, int q, cudaStream_t st) {
-    if (n_ood > MAX_OOD || q > MAX_QUERIES) return -1;
-    k_stir_rlc<<<1, 32, 0, st>>>(tx, sc, commit_idx, n_ood, q);
+    if (a.logN > OPEN_MAX_LOGN || a.ood_offset > MAX_OOD) return -1;
+    // A CTA per 15 rows (one row a warp), at most OPEN_CTAS.
+    const u32 rows = OPEN_WARPS - 1, ctas = std::min(OPEN_CTAS, std::max(1u, (a.q + rows - 1) / rows));
+    k_open<<<ctas, OPEN_THREADS, 0, st>>>(a);
     count_launches(1);
     return 0;
 }

@@ -178,6 +178,8 @@ int launch_tx_init(TxState* tx, const unsigned char* ds, u32 ds_len, unsigned ch
 int launch_constraint_rlc(TxState* tx, ProofScalars* sc, int n_forms, int nwit, int ood, int nvec, cudaStream_t st);
 // PoW: squeeze the 32-byte challenge, grind the minimum nonce, send it.
 int launch_pow(TxState* tx, ProofScalars* sc, u64 threshold, int slot, int hash, cudaStream_t st);
+// The challenge and the search; the nonce (sc->pow_best) is sent by k_open.
+int launch_pow_search(TxState* tx, ProofScalars* sc, u64 threshold, int hash, cudaStream_t st);
 // `count` Ext3 challenges into sc->sc_r[slot ..] (verifier_message_vec).
 int launch_squeeze_challenges(TxState* tx, ProofScalars* sc, int slot, int count, cudaStream_t st);
 // Sends every coefficient of the final folded vector (whir_prover.hpp:360-362).
@@ -203,11 +205,10 @@ struct OpenArgs {
     int r_offset;       // sc->sc_r[r_offset .. r_offset + fold) are the folding randomness
     u32 fold;           // number of folding variables (2^fold columns per vector)
     u32 perm_log_e;     // coset-major rows (see launch_leaves); 0 = natural order
+    int pow_slot;       // >= 0: a PoW search precedes; send its nonce first (recorded in sc->pow_nonces[pow_slot])
+    int rlc_commit;     // stir: the new commitment, whose ood_offset OOD points/values join the STIR combination
 };
 int launch_open(const OpenArgs& a, cudaStream_t st);
-// STIR combination (whir_prover.hpp:283-336): copy the new commitment's OOD
-// points/values into the STIR arrays, squeeze the geometric RLC, update the sum.
-int launch_stir_rlc(TxState* tx, ProofScalars* sc, int commit_idx, int n_ood, int q, cudaStream_t st);
 
 // ---- Covector / sumcheck ---------------------------------------------------------
 // cov[i] = sum_f crlc_f eq(p_f, i) + sum_j crlc_{F+j} z_j^i over 2^logS entries

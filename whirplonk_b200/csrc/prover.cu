@@ -435,7 +435,8 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
         const uint32_t deg = (uint32_t)p.params.field_degree;
         const uint64_t* src[3] = {c.a(0), deg >= 2 ? c.a(1) : nullptr, deg >= 2 ? c.a(2) : nullptr};
         WG_TRY(commit_vectors(c, ci, src, deg, vsize, 1, (int)rc.irs.out_domain, &c.sc()->ood_vals[ci][0], 1));
-        WG_TIMED(c, FAM_POW, launch_pow(c.tx(), c.sc(), rc.pow_threshold, ci, c.p.params.hash, st));
+        // (the opening sends the nonce)
+        WG_TIMED(c, FAM_POW, launch_pow_search(c.tx(), c.sc(), rc.pow_threshold, c.p.params.hash, st));
         // open the previous commitment (the first round: every initial commitment)
         const IrsSchedule& prev = r == 0 ? s.initial : s.rounds[r - 1].irs;
         const CommitBuffers& pb = p.commits[r == 0 ? 0 : ci - 1];
@@ -460,8 +461,9 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
         const uint32_t prev_fold = (uint32_t)(r == 0 ? s.initial_sumcheck.num_rounds : s.rounds[r - 1].sumcheck.num_rounds);
         oa.fold = prev_fold;
         oa.r_offset = r_slot - (int)prev_fold;
+        oa.pow_slot = rc.pow_threshold == ~0ull ? -1 : ci;
+        oa.rlc_commit = ci;
         WG_TIMED(c, FAM_OPEN, launch_open(oa, st));
-        WG_TIMED(c, FAM_TX, launch_stir_rlc(c.tx(), c.sc(), ci, (int)rc.irs.out_domain, (int)prev.in_domain, st));
         CovAccArgs ca{};
         for (int k = 0; k < 3; ++k) ca.cov[k] = c.cov(k);
         ca.size = vsize;
@@ -477,7 +479,7 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
 
     // final vector, PoW, opening, sumcheck
     WG_TIMED(c, FAM_TX, launch_send_vector(c.tx(), c.a(0), c.a(1), c.a(2), vsize, st));
-    WG_TIMED(c, FAM_POW, launch_pow(c.tx(), c.sc(), s.final_pow, (int)(W + s.rounds.size()), c.p.params.hash, st));
+    WG_TIMED(c, FAM_POW, launch_pow_search(c.tx(), c.sc(), s.final_pow, c.p.params.hash, st));
     {
         const bool initial = s.rounds.empty();
         const IrsSchedule& last = initial ? s.initial : s.rounds.back().irs;
@@ -498,6 +500,7 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
         oa.gen = 1;
         oa.stir = 0;
         oa.perm_log_e = lb.perm_log_e;
+        oa.pow_slot = s.final_pow == ~0ull ? -1 : (int)(W + s.rounds.size());
         WG_TIMED(c, FAM_OPEN, launch_open(oa, st));
     }
     if (s.final_sumcheck.num_rounds > 0) WG_TRY(sumcheck(c, s.final_sumcheck, vsize, false, r_slot, false));

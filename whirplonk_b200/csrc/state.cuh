@@ -55,5 +55,6 @@ struct ProofScalars {
 };
 // ProofScalars::counters slots.
 constexpr int CTR_MERKLE_TAIL = 0;  // k_merkle_tail: subtree CTAs finished
+constexpr int CTR_OPEN = 1;         // k_open: CTAs finished
 
 }  // namespace wg

@@ -766,6 +766,7 @@ whirgpu_status whirgpu_zk_prove(whirgpu_ctx* c, whirgpu_zk_witness* w, const whi
         oa.q = (u32)init.in_domain;
         oa.gen = 1;
         oa.stir = 0;
+        oa.pow_slot = -1;
         if (launch_open(oa, st) != 0) return zk_fail(c, WHIRGPU_E_INVALID, "opening launch failed");
     }
     k_zk_taus<<<1, 32, 0, st>>>(txs, zs);
