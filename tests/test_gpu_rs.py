@@ -187,3 +187,25 @@ def test_pipelined_plans_proof_matches_oracle(gpu_ctx, oracle):
     finally:
         L.whirgpu_ntt_clear_plans()
         load_plans()
+
+
+@pytest.mark.parametrize("log_len,log_exp,log_depth,count", [(17, 4, 3, 1), (17, 4, 3, 3), (19, 4, 6, 1), (18, 4, 5, 5),
+                                                             (18, 3, 4, 1)])
+def test_leaf_ring_row_widths(gpu_ctx, oracle, log_len, log_exp, log_depth, count):
+    """From 2^17 rows on the leaves are hashed from a ring of bulk copies: rows
+    of 1 to 8 blocks, one and several matrices, the smallest row count."""
+    v = sample_goldilocks(8800 + log_len + 10 * log_depth + count, count << log_len).reshape(count, -1)
+    roots = rs_commit_batch(gpu_ctx, v, log_exp, log_depth)
+    N = ((1 << log_len) >> log_depth) << log_exp
+    for k in range(count):
+        assert roots[k] == oracle.rs_commit_root(v[k], N, 1 << log_depth), f"vector {k}"
+
+
+def test_leaf_ring_ext3_rows(gpu_ctx, oracle):
+    """A proof whose first round commits 2^17 Ext3 rows."""
+    n, rho = 19, 3
+    params = ProtocolParameters.cli(log_inv_rate=rho)
+    coeffs = sample_goldilocks(93, 1 << n)
+    pts = sample_goldilocks(94, 3 * n).reshape(1, n, 3)
+    ev = np.array(gpu_ctx.mle_evaluate(coeffs, pts), dtype=np.uint64).reshape(1, 3)
+    assert prove_once(n, params, coeffs, pts, ev, ctx=gpu_ctx)[:2] == oracle.prove(n, 4, rho, 100, 20, pts, coeffs, ev)

@@ -127,12 +127,14 @@ int sumcheck_prepare();
 // hash: 0 = BLAKE3, 1 = SHA-256 (the engine a configuration's hash_id selects).
 // perm_log_e > 0: coset-major rows -- leaf k hashes natural row
 // (k >> (logN - perm_log_e)) + ((k mod 2^(logN - perm_log_e)) << perm_log_e).
+// err: device error word (TX_ERR_TIMEOUT), or null.
 int launch_leaves(const u64* planes, u64 N, u32 depth, u32 ncomp, u32* nodes, int hash, cudaStream_t st,
-                  u32 perm_log_e = 0);
+                  u32 perm_log_e = 0, u32* err = nullptr);
+int leaves_prepare();
 // `count` independent matrices: planes and node arrays `plane_stride` /
 // `node_stride` words apart.
 int launch_leaves_batch(const u64* planes, u64 N, u32 depth, u32 ncomp, u32* nodes, u32 count, u64 plane_stride,
-                        u64 node_stride, int hash, cudaStream_t st, u32 perm_log_e = 0);
+                        u64 node_stride, int hash, cudaStream_t st, u32 perm_log_e = 0, u32* err = nullptr);
 // Builds all Merkle levels above the leaves of a 2^logN-leaf tree in `nodes`
 // ([leaves | level 1 | ... | root], 8 words per node).  The CTA that computes
 // the root also performs the transcript step of irs_commit::commit

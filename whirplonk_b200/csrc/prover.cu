@@ -233,7 +233,7 @@ int commit_vectors(const Ctx& c, int ci, const uint64_t* const src[3], uint32_t 
     WG_TIMED(c, FAM_NTT, launch_lde(L, c.st));
     uint32_t* nodes = reinterpret_cast<uint32_t*>(c.ws + cb.nodes);
     WG_TIMED(c, FAM_LEAF, launch_leaves(c.w(cb.planes), cb.N, cb.depth, ncomp, nodes, c.p.params.hash, c.st,
-                                        cb.perm_log_e));
+                                        cb.perm_log_e, &c.tx()->err));
     WG_TIMED(c, FAM_MERKLE, launch_merkle(nodes, cb.logN, c.tx(), c.sc(), ci, n_ood, c.p.params.hash, c.st));
     OodArgs o{};
     for (int k = 0; k < 3; ++k) o.v[k] = src[k] ? src[k] : src[0];
