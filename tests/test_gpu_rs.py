@@ -209,3 +209,32 @@ def test_leaf_ring_ext3_rows(gpu_ctx, oracle):
     pts = sample_goldilocks(94, 3 * n).reshape(1, n, 3)
     ev = np.array(gpu_ctx.mle_evaluate(coeffs, pts), dtype=np.uint64).reshape(1, 3)
     assert prove_once(n, params, coeffs, pts, ev, ctx=gpu_ctx)[:2] == oracle.prove(n, 4, rho, 100, 20, pts, coeffs, ev)
+
+
+def test_commitments_of_concurrent_contexts(gpu_ctx):
+    """Encoder and leaf ring of several contexts at once, their CTAs sharing
+    SMs: every root equals the one computed alone."""
+    import threading
+
+    import torch
+
+    shapes = [(22, 2, 4), (21, 3, 4), (20, 4, 3), (22, 1, 5), (20, 3, 2), (21, 2, 4)]
+    vs = [torch.from_numpy(sample_goldilocks(7100 + i, 1 << ll).view(np.int64)).cuda() for i, (ll, _, _) in enumerate(shapes)]
+    want = [rs_commit_batch(gpu_ctx, None, lx, ld, on_device_ptr=v.data_ptr(), count=1, log_len=ll)
+            for (ll, lx, ld), v in zip(shapes, vs)]
+    bad = []
+
+    def work(i):
+        ll, lx, ld = shapes[i]
+        ctx = Context(0)
+        for _ in range(40):
+            if rs_commit_batch(ctx, None, lx, ld, on_device_ptr=vs[i].data_ptr(), count=1, log_len=ll) != want[i]:
+                bad.append(i)
+        ctx.close()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(shapes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad

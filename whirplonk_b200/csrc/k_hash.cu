@@ -15,6 +15,7 @@
 
 #include "launch.h"
 #include "blake3.cuh"
+#include "i8mma.cuh"
 #include "sha256.cuh"
 #include "state.cuh"
 #include "wtx.cuh"
@@ -153,34 +154,10 @@ __global__ void __launch_bounds__(256, NCOMP == 3 ? 3 : 1) k_leaves(const u64* _
 // loads take no registers, run RING_STAGES blocks ahead and across tiles, which
 // is what k_leaves lacks: its loads ahead cost registers, it issued at 0.69 of
 // the compression rate waiting for them.  Measured on B200, all leaves of an
-// n = 24 rate 1/4 proof (32.8 M compressions): 1208 -> 1047 us, 0.79 of the rate;
-// 3 CTAs of 4 stages 1055 us, 5 of 2 stages 1152 us.
+// n = 24 rate 1/4 proof (32.8 M compressions): 1208 -> 1098 us, 0.76 of the rate;
+// 3 CTAs of 4 stages 1110 us, 5 of 2 stages 100 us more.
 constexpr int RING_WARPS = 8, RING_ROWS = 32 * RING_WARPS, RING_STAGES = 3, RING_CTAS = 4;
 constexpr u32 RING_STAGE_BYTES = 8 * RING_ROWS * 8;
-
-__device__ __forceinline__ u32 ring_smem(const void* p) { return (u32)__cvta_generic_to_shared(p); }
-// Waits for the phase; gives up after about two seconds (a stage takes
-// microseconds) and reports it.
-__device__ __forceinline__ bool ring_wait(u32 bar, u32 parity) {
-    unsigned long long t0 = 0;
-    for (u32 it = 0; it < (1u << 28); ++it) {
-        u32 done;
-        asm volatile("{\n\t.reg .pred p;\n\t"
-                     "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(done)
-                     : "r"(bar), "r"(parity)
-                     : "memory");
-        if (done) return true;
-        if ((it & 63) == 63) {
-            unsigned long long t;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-            if (!t0) t0 = t;
-            else if (t - t0 > 2000000000ull) return false;
-        }
-    }
-    return false;
-}
 
 struct RingArgs {
     const u64* planes;
@@ -196,11 +173,11 @@ __global__ void __launch_bounds__(RING_ROWS + 32, RING_CTAS) k_leaves_ring(const
     extern __shared__ __align__(128) unsigned char ring[];
     __shared__ __align__(8) u64 bars[2 * RING_STAGES];
     const u32 warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const u32 full = ring_smem(bars), empty = full + 8 * RING_STAGES, base = ring_smem(ring);
+    const u32 full = smem_u32(bars), empty = full + 8 * RING_STAGES, base = smem_u32(ring);
     if (threadIdx.x == 0)
         for (u32 s = 0; s < RING_STAGES; ++s) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(full + 8 * s) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(empty + 8 * s), "n"(RING_WARPS) : "memory");
+            mbar_init(full + 8 * s, 1);
+            mbar_init(empty + 8 * s, RING_WARPS);
         }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     __syncthreads();
@@ -212,7 +189,7 @@ __global__ void __launch_bounds__(RING_ROWS + 32, RING_CTAS) k_leaves_ring(const
                 const u64* src = a.planes + (u64)(tile >> a.log_tiles) * a.plane_stride +
                                  (u64)(tile & ((1u << a.log_tiles) - 1)) * RING_ROWS;
                 for (u32 t = 0; t < a.nblocks && ok; ++t) {
-                    ok = ring_wait(empty + 8 * s, ph ^ 1);
+                    ok = mbar_wait(empty + 8 * s, ph ^ 1);
                     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full + 8 * s),
                                  "n"(RING_STAGE_BYTES)
                                  : "memory");
@@ -231,7 +208,7 @@ __global__ void __launch_bounds__(RING_ROWS + 32, RING_CTAS) k_leaves_ring(const
             unsigned cv[8];
             b3_init(cv);
             for (u32 t = 0; t < a.nblocks; ++t) {
-                ok = ok && ring_wait(full + 8 * s, ph);
+                ok = ok && mbar_wait(full + 8 * s, ph);
                 const u64* row = reinterpret_cast<const u64*>(ring + s * RING_STAGE_BYTES) + threadIdx.x;
                 unsigned m[16];
 #pragma unroll
@@ -240,8 +217,12 @@ __global__ void __launch_bounds__(RING_ROWS + 32, RING_CTAS) k_leaves_ring(const
                     m[2 * q] = (unsigned)v;
                     m[2 * q + 1] = (unsigned)(v >> 32);
                 }
+                // The next copies write this stage through the async proxy: the
+                // reads above must have been performed, which an arrival alone
+                // does not say (under load from other kernels it overtook them).
+                fence_async();
                 __syncwarp();
-                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(empty + 8 * s) : "memory");
+                if (lane == 0) mbar_arrive(empty + 8 * s);
                 if (++s == RING_STAGES) s = 0, ph ^= 1;
                 const unsigned flags = (t == 0 ? B3_CHUNK_START : 0u) | (t + 1 == a.nblocks ? (B3_CHUNK_END | B3_ROOT) : 0u);
                 b3_compress(cv, m, flags);
