@@ -793,6 +793,8 @@ size_t cov_acc_scratch_bytes(u64 size, int n_points) {
 int launch_cov_accumulate(const CovAccArgs& a, cudaStream_t st) {
     const int npts = a.n_ext + a.n_base;
     if (npts == 0 || a.size == 0) return 0;
+    const int rc = launch_cov_gemm(a, st);
+    if (rc != 1) return rc;
     const u32 hc = ca_hi_count(a.size);
     E3* tab = reinterpret_cast<E3*>(a.scratch);
     const size_t tab_bytes = ((size_t)(1u << CA_LO) + hc) * (size_t)npts * sizeof(E3);

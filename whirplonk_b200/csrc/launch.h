@@ -243,8 +243,14 @@ struct CovAccArgs {
     ProofScalars* sc;
     void* scratch;
     int ext2;
+    void* big;          // scratch of the contraction form (any, may be null)
+    size_t big_bytes;
+    u32* err;           // device error word (TX_ERR_TIMEOUT), or null
 };
 int launch_cov_accumulate(const CovAccArgs& a, cudaStream_t st);
+// The same by 8-bit contraction (k_cov_gemm.cu); 1: does not apply.
+int launch_cov_gemm(const CovAccArgs& a, cudaStream_t st);
+int cov_gemm_prepare();
 size_t cov_acc_scratch_bytes(u64 size, int n_points);
 
 struct SumcheckArgs {

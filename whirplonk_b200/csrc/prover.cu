@@ -472,6 +472,9 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
         ca.sc = c.sc();
         ca.scratch = ws + p.off_cov_scratch;
         ca.ext2 = p.params.field_degree == 2;
+        ca.big = ws + p.off_tmp;  // the LDE scratch: free between commitments
+        ca.big_bytes = p.off_sc_scratch - p.off_tmp;
+        ca.err = &c.tx()->err;
         WG_TIMED(c, FAM_COV, launch_cov_accumulate(ca, st));
         WG_TRY(sumcheck(c, rc.sumcheck, vsize, false, r_slot, true));
         vsize >>= rc.sumcheck.num_rounds;
