@@ -273,6 +273,7 @@ __global__ void __launch_bounds__(256) k_tsc_rounds(TscRoundArgs a) {
         ProofScalars* sc = a.sc;
         WarpTx wt;
         wtx_load(wt, a.tx);
+        E3 sum = sc->sum;
         for (u32 r = 0; r < a.k; ++r) {
             const u32 h = nb >> (r + 1);
             E3 c0 = e3_zero(), c2 = e3_zero();
@@ -284,18 +285,18 @@ __global__ void __launch_bounds__(256) k_tsc_rounds(TscRoundArgs a) {
             }
             c0 = wtx_sum(c0);
             c2 = wtx_sum(c2);
-            wtx_message_t(wt, c0);
-            wtx_message_t(wt, c2);
+            wtx_absorb2_t(wt, c0, c2);
             const E3 rn = wtx_challenge_t(wt);
+            wtx_narg_t(wt, c0);
+            wtx_narg_t(wt, c2);
+            const E3 c1 = e3_sub(e3_sub(sum, e3_add(c0, c0)), c2);
+            sum = e3_add(e3_mul(e3_add(e3_mul(c2, rn), c1), rn), c0);
             if (lane == 0) {
-                const E3 c1 = e3_sub(e3_sub(sc->sum, e3_add(c0, c0)), c2);
                 sc->c0 = c0;
                 sc->c2 = c2;
                 sc->sc_r[a.r_slot + r] = rn;
-                sc->sum = e3_add(e3_mul(e3_add(e3_mul(c2, rn), c1), rn), c0);
                 rs[r] = rn;
             }
-            __syncwarp();
             for (u32 v = lane; v < (u32)a.T * h; v += 32) {
                 const u32 t = v / h, i = v % h;
                 E3& zl = Z[t * nb + i];
@@ -305,6 +306,7 @@ __global__ void __launch_bounds__(256) k_tsc_rounds(TscRoundArgs a) {
             }
             __syncwarp();
         }
+        if (lane == 0) sc->sum = sum;
         wtx_store(wt, a.tx);
     }
     __syncthreads();

@@ -27,50 +27,63 @@ struct WarpTx {
 
 __device__ __forceinline__ unsigned wtx_lane() { return threadIdx.x & 31; }
 
-__device__ __forceinline__ u64 rotl64_var(u64 v, unsigned s) { return s ? ((v << s) | (v >> (64 - s))) : v; }
-
-// Source lane of pi for lane (X, Y): pi moves A[x][y] to (y, 2x + 3y), so lane
-// (X, Y) receives from (3 (Y - 3X) mod 5, X).
-__device__ __forceinline__ unsigned keccak_pi_src(unsigned x, unsigned y) {
-    return ((5 + 3 * ((y + 15 - 3 * x) % 5)) % 5) + 5 * x;
+// The rho offsets of ten consecutive lanes from l0, six bits each.
+__host__ __device__ constexpr u64 keccak_rho_pack(int l0) {
+    u64 v = 0;
+    for (int i = 0; i < 10 && l0 + i < 25; ++i) v |= (u64)keccak_rho((l0 + i) % 5, (l0 + i) / 5) << (6 * i);
+    return v;
 }
 
-// Keccak-f[1600] with state word l in lane l (lanes 25..31 carry a dummy).
-// Lane (x, y) = x + 5 y.  Each lane rotates its own word (rho), then fetches
-// the three pi-permuted words chi needs -- B[X][Y], B[X+1][Y], B[X+2][Y] --
-// straight from their source lanes: three shuffle stages per round (theta's
-// column sums, theta's D, pi + chi).
+// Keccak-f[1600] with state word l in lane l.  Lane (x, y) = x + 5 y.  Each lane
+// rotates its own word (rho), then fetches the three pi-permuted words chi needs
+// -- B[X][Y], B[X+1][Y], B[X+2][Y] -- straight from their source lanes: three
+// shuffle stages per round (theta's column sums, theta's D, pi + chi).  pi moves
+// A[x][y] to (y, 2x + 3y), so lane (X, Y) receives from ((X + 3Y) mod 5, X).
+// Nothing reads lanes 25..31.
+//
+// Bound by the 18 shuffles a round (~9 cycles each from one warp).  The words are
+// kept as halves, so that a rotation is two selects and two funnel shifts (64-bit
+// shifts: +4 %), and the lane's sources are a few instructions (25 compares for
+// the offset and a dozen remainders: +~0.3 us a call).
 static __device__ __noinline__ u64 keccak_f1600_warp(u64 a) {
     const unsigned l = wtx_lane();
-    const bool live = l < 25;
-    const unsigned x = live ? l % 5 : 0, y = live ? l / 5 : 0;
+    auto div5 = [](unsigned v) { return (v * 13) >> 6; };  // v < 32
+    auto mod5 = [](unsigned v) { return v >= 5 ? v - 5 : v; };  // v < 10
+    const unsigned y = div5(l), x = l - 5 * y;
+    const unsigned v = x + 3 * y, s = v - 5 * div5(v);
     unsigned th[4];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) th[k] = live ? x + 5 * ((y + 1 + k) % 5) : l;
-    const unsigned cl = live ? (x + 4) % 5 + 5 * y : l, cr = live ? (x + 1) % 5 + 5 * y : l;
-    const unsigned p0 = live ? keccak_pi_src(x, y) : l;
-    const unsigned p1 = live ? keccak_pi_src((x + 1) % 5, y) : l;
-    const unsigned p2 = live ? keccak_pi_src((x + 2) % 5, y) : l;
-    unsigned rot = 0;
-#pragma unroll
-    for (int yy = 0; yy < 5; ++yy)
-#pragma unroll
-        for (int xx = 0; xx < 5; ++xx)
-            if (live && x == (unsigned)xx && y == (unsigned)yy) rot = keccak_rho(xx, yy);
+    for (int k = 0; k < 4; ++k) th[k] = x + 5 * mod5(y + 1 + k);
+    const unsigned x1 = mod5(x + 1), cl = mod5(x + 4) + 5 * y, cr = x1 + 5 * y;
+    const unsigned p0 = s + 5 * x, p1 = mod5(s + 1) + 5 * x1, p2 = mod5(s + 2) + 5 * mod5(x + 2);
+    const unsigned g = l < 10 ? 0u : l < 20 ? 10u : 20u;
+    const u64 pack = l < 10 ? keccak_rho_pack(0) : l < 20 ? keccak_rho_pack(10) : keccak_rho_pack(20);
+    const unsigned rot = (unsigned)(pack >> (6 * ((l - g) % 10))) & 63;
+    const bool swap = rot & 32;
+    const unsigned rs = rot & 31, mask = l == 0 ? ~0u : 0u;
+    unsigned lo = (unsigned)a, hi = (unsigned)(a >> 32);
 #pragma unroll 1
     for (int round = 0; round < 24; ++round) {
-        u64 c = a;
+        const u64 rc = KECCAK_RC[round];
+        unsigned s0[4], s1[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) c ^= __shfl_sync(0xFFFFFFFFu, a, th[k]);
-        const u64 d = __shfl_sync(0xFFFFFFFFu, c, cl) ^ rotl64_var(__shfl_sync(0xFFFFFFFFu, c, cr), 1);
-        a ^= d;
-        const u64 r = rotl64_var(a, rot);
-        const u64 b0 = __shfl_sync(0xFFFFFFFFu, r, p0), b1 = __shfl_sync(0xFFFFFFFFu, r, p1),
-                  b2 = __shfl_sync(0xFFFFFFFFu, r, p2);
-        a = b0 ^ (~b1 & b2);
-        if (l == 0) a ^= KECCAK_RC[round];
+        for (int k = 0; k < 4; ++k) {
+            s0[k] = __shfl_sync(0xFFFFFFFFu, lo, th[k]);
+            s1[k] = __shfl_sync(0xFFFFFFFFu, hi, th[k]);
+        }
+        const unsigned c0 = (lo ^ s0[0] ^ s0[1]) ^ s0[2] ^ s0[3], c1 = (hi ^ s1[0] ^ s1[1]) ^ s1[2] ^ s1[3];
+        const unsigned e0 = __shfl_sync(0xFFFFFFFFu, c0, cr), e1 = __shfl_sync(0xFFFFFFFFu, c1, cr);
+        const unsigned g0 = __shfl_sync(0xFFFFFFFFu, c0, cl), g1 = __shfl_sync(0xFFFFFFFFu, c1, cl);
+        const unsigned t0 = lo ^ g0 ^ __funnelshift_l(e1, e0, 1), t1 = hi ^ g1 ^ __funnelshift_l(e0, e1, 1);
+        const unsigned u0 = swap ? t1 : t0, u1 = swap ? t0 : t1;
+        const unsigned r0 = __funnelshift_l(u1, u0, rs), r1 = __funnelshift_l(u0, u1, rs);
+        const unsigned a0 = __shfl_sync(0xFFFFFFFFu, r0, p0), a1 = __shfl_sync(0xFFFFFFFFu, r1, p0);
+        const unsigned b0 = __shfl_sync(0xFFFFFFFFu, r0, p1), b1 = __shfl_sync(0xFFFFFFFFu, r1, p1);
+        const unsigned d0 = __shfl_sync(0xFFFFFFFFu, r0, p2), d1 = __shfl_sync(0xFFFFFFFFu, r1, p2);
+        lo = (a0 ^ (~b0 & d0)) ^ ((unsigned)rc & mask);
+        hi = (a1 ^ (~b1 & d1)) ^ ((unsigned)(rc >> 32) & mask);
     }
-    return a;
+    return (u64)hi << 32 | lo;
 }
 
 __device__ __forceinline__ void wtx_load(WarpTx& t, const TxState* g) {
@@ -119,21 +132,38 @@ __device__ __forceinline__ void wtx_absorb_byte(WarpTx& t, u8 v) {
         t.hpos = 0;
     }
 }
-__device__ __forceinline__ void wtx_absorb_words(WarpTx& t, const u64* w, unsigned nw) {
+// The first nw (<= N) words of w.  At a word boundary every word goes to its lane
+// in one pass; word by word, each with its own test for a full block, took ~190
+// cycles a word on B200.
+template <int N>
+__device__ __forceinline__ void wtx_absorb_words(WarpTx& t, const u64 (&w)[N], unsigned nw) {
+    static_assert(8 * N <= TX_RATE, "at most one block boundary");
+    constexpr unsigned RW = TX_RATE / 8;
     t.has_reader = 0;
-    for (unsigned i = 0; i < nw; ++i) {
-        const u64 v = w[i];
-        if ((t.hpos & 7) == 0) {
-            if (wtx_lane() == (t.hpos >> 3)) t.h ^= v;
-            t.hpos += 8;
-            if (t.hpos == TX_RATE) {
-                t.h = keccak_f1600_warp(t.h);
-                t.hpos = 0;
+    if ((t.hpos & 7) == 0) {
+        const unsigned at = t.hpos >> 3, k = wtx_lane() - at;  // this lane takes word k of the block
+        u64 v = 0, next = 0;
+#pragma unroll
+        for (unsigned i = 0; i < N; ++i)
+            if (i < nw) {
+                if (k == i) v = w[i];
+                if (k + RW == i) next = w[i];
             }
-        } else {
-#pragma unroll 1
-            for (int b = 0; b < 8; ++b) wtx_absorb_byte(t, (u8)(v >> (8 * b)));
+        if (wtx_lane() < RW) t.h ^= v;
+        t.hpos += 8 * nw;
+        if (t.hpos >= TX_RATE) {
+            t.h = keccak_f1600_warp(t.h) ^ next;
+            t.hpos -= TX_RATE;
         }
+        return;
+    }
+#pragma unroll 1
+    for (unsigned i = 0; i < 8 * nw; ++i) {
+        u64 v = 0;
+#pragma unroll
+        for (unsigned q = 0; q < N; ++q)
+            if (q == i >> 3) v = w[q];
+        wtx_absorb_byte(t, (u8)(v >> (8 * (i & 7))));
     }
 }
 __device__ __forceinline__ void wtx_absorb_bytes(WarpTx& t, const u8* src, unsigned n) {
@@ -202,24 +232,38 @@ __device__ __forceinline__ void wtx_squeeze_bytes(WarpTx& t, u8* dst, unsigned n
     __syncwarp();
 }
 
-__device__ __forceinline__ void wtx_narg_append(WarpTx& t, const u8* src, unsigned n) {
-    if (t.narg_len + n > t.narg_cap) {
+// The first nw (<= N) words of w to the proof string, lane i word i.
+template <int N>
+__device__ __forceinline__ void wtx_narg_words(WarpTx& t, const u64 (&w)[N], unsigned nw) {
+    if (t.narg_len + 8 * nw > t.narg_cap) {
         t.err |= TX_ERR_NARG_OVERFLOW;
         return;
     }
     const unsigned l = wtx_lane();
-    for (unsigned i = l; i < n; i += 32) t.narg[t.narg_len + i] = src[i];
-    t.narg_len += n;
+    u64 v = 0;
+#pragma unroll
+    for (unsigned i = 0; i < N; ++i)
+        if (l == i) v = w[i];
+    u8* dst = t.narg + t.narg_len + 8 * l;
+    if (l < nw) {
+        if ((reinterpret_cast<u64>(dst) & 7) == 0) {
+            *reinterpret_cast<u64*>(dst) = v;
+        } else {
+#pragma unroll 1
+            for (int b = 0; b < 8; ++b) dst[b] = (u8)(v >> (8 * b));
+        }
+    }
+    t.narg_len += 8 * nw;
 }
-__device__ __forceinline__ void wtx_message_words(WarpTx& t, const u64* w, unsigned nw) {
+template <int N>
+__device__ __forceinline__ void wtx_message_words(WarpTx& t, const u64 (&w)[N], unsigned nw = N) {
     wtx_absorb_words(t, w, nw);
-    wtx_narg_append(t, reinterpret_cast<const u8*>(w), 8 * nw);
+    wtx_narg_words(t, w, nw);
 }
-__device__ __forceinline__ void wtx_message_e3(WarpTx& t, E3 v) {
-    u64 w[3] = {v.c0, v.c1, v.c2};
-    wtx_message_words(t, w, 3);
+__device__ __forceinline__ void wtx_message_u64(WarpTx& t, u64 v) {
+    const u64 w[1] = {v};
+    wtx_message_words(t, w);
 }
-__device__ __forceinline__ void wtx_message_u64(WarpTx& t, u64 v) { wtx_message_words(t, &v, 1); }
 
 // 40 squeezed bytes as a LE integer mod p (five words folded from the top).
 __device__ __forceinline__ u64 wtx_challenge_base(WarpTx& t) {
@@ -232,25 +276,20 @@ __device__ __forceinline__ u64 wtx_challenge_base(WarpTx& t) {
 }
 
 // ncomp (<= 3) consecutive base-field challenges, lane-parallel when their
-// 40 ncomp bytes start word-aligned inside the current reader block: lane k <
-// 5 ncomp takes squeezed word k and scales it by 2^(64 (k mod 5)) mod p (the
-// powers are 1, 2^32 - 1, p - 2^32, 1, 2^32 - 1), and lane c sums the five
-// terms of challenge c -- the integer sum_i w_i 2^(64 i) mod p that the
-// word-by-word fold above computes.  Otherwise the challenges are squeezed
-// word by word.  Returns challenge c in component c.
+// 40 ncomp bytes start word-aligned inside the current reader block: lane c
+// gathers the five words of challenge c and folds them as above.  Otherwise the
+// challenges are squeezed word by word.  Returns challenge c in component c.
 __device__ __forceinline__ E3 wtx_challenges(WarpTx& t, u32 ncomp) {
     wtx_reader(t);
     const unsigned l = wtx_lane();
     if ((t.rpos & 7) == 0 && t.rpos + 40 * ncomp <= TX_RATE) {
-        const u32 k = l < 5 * ncomp ? l : 0;
-        const u64 w = __shfl_sync(0xFFFFFFFFu, t.r, (t.rpos >> 3) + k);
-        const u32 i = k % 5;
-        const u64 scale = (i == 0 || i == 3) ? 1ull : (i == 2 ? GL_P - (1ull << 32) : GL_EPS);
-        const u64 term = gl_mul(w, scale);
-        const u32 src = l < ncomp ? 5 * l : 0;
-        u64 s = __shfl_sync(0xFFFFFFFFu, term, src);
-#pragma unroll 1
-        for (u32 q = 1; q < 5; ++q) s = gl_add(s, __shfl_sync(0xFFFFFFFFu, term, src + q));
+        const u32 src = (t.rpos >> 3) + (l < ncomp ? 5 * l : 0);
+        u64 w[5];
+#pragma unroll
+        for (u32 q = 0; q < 5; ++q) w[q] = __shfl_sync(0xFFFFFFFFu, t.r, src + q);
+        u64 s = gl_reduce(w[4], 0);
+#pragma unroll
+        for (int q = 3; q >= 0; --q) s = gl_reduce(w[q], s);
         t.rpos += 40 * ncomp;
         const u64 c0 = __shfl_sync(0xFFFFFFFFu, s, 0);
         const u64 c1 = __shfl_sync(0xFFFFFFFFu, s, 1);
@@ -274,17 +313,26 @@ __device__ __forceinline__ E3 wtx_challenge_e3(WarpTx& t) { return wtx_challenge
 __device__ __forceinline__ E3 wtx_challenge_t(WarpTx& t) {
     return wtx_challenges(t, t.deg == 1 ? 1u : (t.deg == 2 ? 2u : 3u));
 }
-__device__ __forceinline__ void wtx_message_t(WarpTx& t, E3 v) {
-    if (t.deg == 1) {
-        if (v.c1 | v.c2) t.err |= TX_ERR_FIELD;  // outside the base field: caller input was not base-field
-        wtx_message_u64(t, v.c0);
-    } else if (t.deg == 2) {
-        if (v.c2) t.err |= TX_ERR_FIELD;  // outside GoldilocksExt2's (c0, c1)
-        u64 w[2] = {v.c0, v.c1};
-        wtx_message_words(t, w, 2);
-    } else {
-        wtx_message_e3(t, v);
-    }
+__device__ __forceinline__ void wtx_check_t(WarpTx& t, const E3& v) {  // caller input outside the target field
+    if ((t.deg == 1 && v.c1) || (t.deg <= 2 && v.c2)) t.err |= TX_ERR_FIELD;
+}
+__device__ __forceinline__ void wtx_narg_t(WarpTx& t, const E3& v) {
+    const u64 w[3] = {v.c0, v.c1, v.c2};
+    wtx_narg_words(t, w, t.deg);
+}
+__device__ __forceinline__ void wtx_message_t(WarpTx& t, const E3& v) {
+    wtx_check_t(t, v);
+    const u64 w[3] = {v.c0, v.c1, v.c2};
+    wtx_message_words(t, w, t.deg);
+}
+// Two consecutive messages, absorbed in one pass and not yet in the proof string:
+// the caller appends them (wtx_narg_t) once the challenge has been handed on.
+__device__ __forceinline__ void wtx_absorb2_t(WarpTx& t, const E3& x, const E3& y) {
+    wtx_check_t(t, x);
+    wtx_check_t(t, y);
+    const bool d1 = t.deg == 1, d2 = t.deg == 2;
+    const u64 w[6] = {x.c0, d1 ? y.c0 : x.c1, d2 ? y.c0 : x.c2, d2 ? y.c1 : y.c0, y.c1, y.c2};
+    wtx_absorb_words(t, w, 2 * t.deg);
 }
 
 // geometric_challenge (geometric_challenge.hpp:39-44): [] / [1] / squeeze x ->
