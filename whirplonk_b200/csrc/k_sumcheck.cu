@@ -158,8 +158,7 @@ __device__ __forceinline__ void sc_round_finish(const ScKernelArgs& a, E3 c0, E3
         ProofScalars* sc = a.sc;
         WarpTx t;
         wtx_load(t, a.tx);
-        wtx_message_t(t, C0);
-        wtx_message_t(t, C2);
+        wtx_absorb2_t(t, C0, C2);
         if (a.pow_threshold != ~0ull) {
             // PoW follows in-stream (ordered windows, then k_sc_after_pow).
             wtx_squeeze_bytes(t, sc->pow_ch, 32);
@@ -180,6 +179,8 @@ __device__ __forceinline__ void sc_round_finish(const ScKernelArgs& a, E3 c0, E3
                 sc->sum = e3_add(ef_mul(e3_add(ef_mul(C2, rn, x2), c1), rn, x2), C0);
             }
         }
+        wtx_narg_t(t, C0);
+        wtx_narg_t(t, C2);
         wtx_store(t, a.tx);
         if (threadIdx.x == 0) *a.counter = 0;
     }
@@ -282,131 +283,219 @@ __global__ void k_sc_after_pow(TxState* tx, ProofScalars* sc, int r_slot) {
 }
 
 // ---------------------------------------------------------------------------
-// Small sumchecks (size <= SC_SMALL_MAX, no round PoW): all rounds of one
-// sumcheck, and the fold after the last one, in ONE CTA.  Round t folds with
-// the previous challenge on load exactly as k_sumcheck_round does; warp 0
-// carries the transcript across the rounds; __syncthreads orders the rounds.
-// This replaces a chain of grid launches whose fixed cost dominates at these
-// sizes.
+// Sumchecks of up to 2^15 elements (no round PoW): all rounds of one sumcheck,
+// and the fold after the last one, in one launch of a cluster of C CTAs.
+//
+// CTA c owns the elements i = c (mod C): i and i + s/2 have the same owner in
+// every round (while s/2 >= C), so the folds stay in the CTA's shared memory and
+// only the two sums and the challenge cross CTAs (distributed shared memory,
+// two cluster barriers a round).  A warp of its own in CTA 0 runs the transcript;
+// it updates the claimed sum and appends to the proof string while the others
+// fold.
+//
+// Bound by the round's chain, ~11 k cycles: fold and sums 3-4 k (one element a
+// lane pair: the latency of ~600 instructions), reduction 0.7 k, the transcript's
+// absorb, permutation and challenge 5-6 k.  All sumchecks of a proof on B200,
+// against a launch a round above 2^12 and one CTA over L2 below (one thread per
+// pair, the transcript's warp folding too): n = 12 151 -> 125 us, n = 16 221 -> 163,
+// n = 18 287 -> 212.  Clusters of 4: 2-5 % slower; 512 threads: 4-6 %; one CTA up to
+// 2^10 the same as the cluster.  Above 2^15 the vectors no longer fit a cluster of 8.
 // ---------------------------------------------------------------------------
-constexpr u64 SC_SMALL_MAX = 1ull << 12;
-// 512 threads leave the kernel 128 registers a thread: at 1024 its 192-bit
-// accumulators and the transcript state spilled to local memory.
-constexpr int SC_SMALL_THREADS = 512;
-constexpr int SC_SMALL_WARPS = SC_SMALL_THREADS / 32;
+constexpr u64 SC_SMALL_MAX = 1ull << 15;
+constexpr int SC_CL = 8;                // CTAs of a cluster
+constexpr u64 SC_CL_MIN = 1ull << 9;  // fewer elements: one CTA
+constexpr int SC_CL_THREADS = 256;   // folding threads of a CTA; one more warp for the transcript
 
-struct ScSmallArgs {
+struct ScClusterArgs {
     const u64* a_base;  // base-field coefficients (first sumcheck) or null
     u64* a[3];
     u64* b[3];
-    u64 size;           // size of round 0
+    u32 size;           // elements of round 0
     int rounds, r_slot, fold_after;
     TxState* tx;
     ProofScalars* sc;
     int ext2;
 };
 
-__global__ void __launch_bounds__(SC_SMALL_THREADS) k_sumcheck_small(ScSmallArgs a) {
-    __shared__ E3 red[2][SC_SMALL_WARPS];
-    __shared__ E3 rsh;  // the round's challenge, handed from warp 0 to the CTA
-    ProofScalars* sc = a.sc;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+template <int C>
+__device__ __forceinline__ void cluster_sync_all() {
+    if constexpr (C == 1) {
+        __syncthreads();
+    } else {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+}
+// Stores v to the word of CTA `rank` that corresponds to this CTA's *p.
+template <int C>
+__device__ __forceinline__ void cluster_store(u64* p, u32 rank, u64 v) {
+    if constexpr (C == 1) {
+        *p = v;
+    } else {
+        u32 addr;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((u32)__cvta_generic_to_shared(p)), "r"(rank));
+        asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+    }
+}
+
+// The value of the even lane of this lane's pair.
+__device__ __forceinline__ u64 pair_even(u64 v) { return __shfl_sync(0xFFFFFFFFu, v, threadIdx.x & 30); }
+
+template <int C>
+__global__ void __launch_bounds__(SC_CL_THREADS + 32, 1) k_sumcheck_cluster(const __grid_constant__ ScClusterArgs a) {
+    extern __shared__ u64 vec[];  // planes a0 a1 a2 b0 b1 b2 of this CTA's elements
+    __shared__ u64 part[3][SC_CL_THREADS];
+    __shared__ u64 xsum[C][6];    // CTA 0: every CTA's sums (c0, c2)
+    __shared__ u64 rsh[5];        // the round's challenge, ready for folding (FoldR)
+    const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const u32 rank = C == 1 ? 0 : blockIdx.x;
+    const bool worker = tid < SC_CL_THREADS;
+    const bool chain = !worker && rank == 0;  // the transcript's warp
+    const u32 len = a.size / C;
+    auto ld = [&](u32 p, u32 i) { return E3{vec[p * len + i], vec[(p + 1) * len + i], vec[(p + 2) * len + i]}; };
+    auto st = [&](u32 p, u32 i, const E3& v) {
+        vec[p * len + i] = v.c0;
+        vec[(p + 1) * len + i] = v.c1;
+        vec[(p + 2) * len + i] = v.c2;
+    };
     WarpTx wt;
     E3 sum{};
-    if (warp == 0) {
+    if (chain) {
         wtx_load(wt, a.tx);
-        sum = sc->sum;
+        sum = a.sc->sum;
     }
-    for (int t = 0; t <= a.rounds; ++t) {
-        const bool last = t == a.rounds;  // only the trailing fold
-        if (last && !a.fold_after) break;
-        const u64 size = a.size >> t;
-        const bool fold = t > 0;
-        const bool base = a.a_base && t <= 1;
-        const FoldR r = fold_r(fold ? rsh : e3_zero());
-        ScKernelArgs k{};
-        k.a_base = base ? a.a_base : nullptr;
-        for (int c = 0; c < 3; ++c) { k.a_in[c] = a.a[c]; k.a_out[c] = a.a[c]; k.b[c] = a.b[c]; }
-        k.size = size;
-        k.fold = fold;
-        k.ext2 = a.ext2;
-        if (last) {  // fold only
-            for (u64 i = threadIdx.x; i < size; i += blockDim.x) {
-                st3(k.a_out, i, load_a(k, i, r));
-                st3(k.b, i, load_b(k, i, r));
+    if (C > 1) cluster_sync_all<C>();  // every CTA runs before any stores to another
+    for (int t = 0; t < a.rounds; ++t) {
+        const u32 n = len >> t, half = n >> 1;  // elements here this round
+        if (worker) {
+            // Two lanes a pair (i, i + half): the even one folds the low elements and
+            // sums c0 = a_l b_l, the odd one the high ones and c2 = (a_h - a_l)(b_h - b_l).
+            E3AccL c{};
+            const FoldR r{rsh[0], rsh[1], rsh[2], rsh[3], rsh[4]};
+            const bool odd = tid & 1;
+            for (u32 j0 = warp * 32; j0 < n; j0 += SC_CL_THREADS) {
+                const bool on = j0 + lane < n;
+                const u32 i = (on ? (j0 + lane) >> 1 : 0) + (odd ? half : 0);
+                E3 x, y;
+                if (t == 0) {
+                    const u64 g = (u64)i * C + rank;
+                    x = a.a_base ? e3_base(a.a_base[g]) : ld3(a.a, g);
+                    y = ld3(a.b, g);
+                } else {
+                    x = fold_e3(ld(0, i), ld(0, i + n), r, a.ext2);
+                    y = fold_e3(ld(3, i), ld(3, i + n), r, a.ext2);
+                }
+                if (on) {
+                    st(0, i, x);
+                    st(3, i, y);
+                }
+                const E3 xl{pair_even(x.c0), pair_even(x.c1), pair_even(x.c2)};
+                const E3 yl{pair_even(y.c0), pair_even(y.c1), pair_even(y.c2)};
+                if (odd) {
+                    x = e3_sub(x, xl);
+                    y = e3_sub(y, yl);
+                }
+                if (on) accl_mac(c, x, y);
             }
-            break;
-        }
-        const u64 half = size >> 1;
-        E3AccL c0{}, c2{};
-        for (u64 i = threadIdx.x; i < half; i += blockDim.x) {
-            if (base && !fold) {
-                const u64 al = a.a_base[i], ah = a.a_base[i + half];
-                const E3 bl = ld3(k.b, i), bh = ld3(k.b, i + half);
-                accl_mac_base(c0, al, bl);
-                accl_mac_base(c2, gl_sub(ah, al), e3_sub(bh, bl));
-            } else {
-                const E3 al = load_a(k, i, r), bl = load_b(k, i, r);
-                if (fold) { st3(k.a_out, i, al); st3(k.b, i, bl); }
-                accl_mac(c0, al, bl);
-                const E3 ah = load_a(k, i + half, r), bh = load_b(k, i + half, r);
-                if (fold) { st3(k.a_out, i + half, ah); st3(k.b, i + half, bh); }
-                accl_mac(c2, e3_sub(ah, al), e3_sub(bh, bl));
+            const E3 w = ef_fix(accl_reduce(c), a.ext2);
+            part[0][tid] = w.c0;
+            part[1][tid] = w.c1;
+            part[2][tid] = w.c2;
+            asm volatile("bar.sync 1, %0;" ::"n"(SC_CL_THREADS) : "memory");
+            if (warp < 3) {  // a warp per component; even lanes c0, odd lanes c2
+                u64 v = part[warp][lane];
+#pragma unroll
+                for (u32 k = 32; k < SC_CL_THREADS; k += 32) v = gl_add(v, part[warp][lane + k]);
+#pragma unroll
+                for (int o = 16; o > 1; o >>= 1) v = gl_add(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+                if (lane < 2) cluster_store<C>(&xsum[rank][warp + 3 * lane], 0, v);
             }
         }
-        // Both sums in one barrier: warp partials to shared memory, then warp 0
-        // adds them lane-parallel (field sums are exact, so order is free).
-        const E3 w0 = e3_warp_sum(ef_fix(accl_reduce(c0), a.ext2));
-        const E3 w2 = e3_warp_sum(ef_fix(accl_reduce(c2), a.ext2));
-        if (lane == 0) {
-            red[0][warp] = w0;
-            red[1][warp] = w2;
+        cluster_sync_all<C>();
+        E3 C0{}, C2{}, rn{};
+        if (chain) {
+            u64 v = 0;
+            if (lane < 6)
+                for (u32 c = 0; c < C; ++c) v = gl_add(v, xsum[c][lane]);
+            auto get = [&](int k) { return __shfl_sync(0xFFFFFFFFu, v, k); };
+            C0 = E3{get(0), get(1), get(2)};
+            C2 = E3{get(3), get(4), get(5)};
+            wtx_absorb2_t(wt, C0, C2);
+            rn = wtx_challenge_t(wt);
+            const FoldR r = fold_r(rn);
+            if (lane < C) {  // a lane per CTA
+                cluster_store<C>(&rsh[0], lane, r.r0);
+                cluster_store<C>(&rsh[1], lane, r.r1);
+                cluster_store<C>(&rsh[2], lane, r.r2);
+                cluster_store<C>(&rsh[3], lane, r.r1d);
+                cluster_store<C>(&rsh[4], lane, r.r2d);
+            }
         }
-        __syncthreads();
-        if (warp == 0) {
-            const int nwarps = (int)(blockDim.x >> 5);
-            const E3 C0 = e3_warp_sum(lane < nwarps ? red[0][lane] : e3_zero());
-            const E3 C2 = e3_warp_sum(lane < nwarps ? red[1][lane] : e3_zero());
-            wtx_message_t(wt, C0);
-            wtx_message_t(wt, C2);
-            const E3 rn = wtx_challenge_t(wt);
+        cluster_sync_all<C>();
+        if (chain) {  // beside the others' folds
+            wtx_narg_t(wt, C0);
+            wtx_narg_t(wt, C2);
             const bool x2 = wt.deg == 2;
             const E3 c1 = e3_sub(e3_sub(sum, e3_add(C0, C0)), C2);
             sum = e3_add(ef_mul(e3_add(ef_mul(C2, rn, x2), c1), rn, x2), C0);
             if (lane == 0) {
-                sc->c0 = C0;
-                sc->c2 = C2;
-                sc->sc_r[a.r_slot + t] = rn;
-                rsh = rn;
+                a.sc->c0 = C0;
+                a.sc->c2 = C2;
+                a.sc->sc_r[a.r_slot + t] = rn;
             }
         }
-        __syncthreads();
     }
-    if (warp == 0) {
-        if (lane == 0) sc->sum = sum;
+    if (worker && a.fold_after) {
+        const FoldR r{rsh[0], rsh[1], rsh[2], rsh[3], rsh[4]};
+        const u32 n = len >> a.rounds;
+        for (u32 i = tid; i < n; i += SC_CL_THREADS) {
+            const u64 g = (u64)i * C + rank;
+            st3(a.a, g, fold_e3(ld(0, i), ld(0, i + n), r, a.ext2));
+            st3(a.b, g, fold_e3(ld(3, i), ld(3, i + n), r, a.ext2));
+        }
+    }
+    if (chain) {
+        if (lane == 0) a.sc->sum = sum;
         wtx_store(wt, a.tx);
     }
+}
+
+static int sumcheck_cluster_prepare() {
+    const size_t cl = SC_SMALL_MAX / SC_CL * 48, one = SC_CL_MIN * 48;
+    return cudaFuncSetAttribute(k_sumcheck_cluster<SC_CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl) == cudaSuccess &&
+                   cudaFuncSetAttribute(k_sumcheck_cluster<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one) == cudaSuccess
+               ? 0
+               : -1;
 }
 
 int launch_sumcheck_small(const SumcheckArgs& s, int rounds, int fold_after, cudaStream_t st) {
     if (s.size > SC_SMALL_MAX || s.pow_threshold != ~0ull || rounds < 1) return 1;  // not this path
     if ((s.size >> rounds) < 1) return -1;
-    ScSmallArgs a{};
+    // The last round's halves still split over the cluster.
+    const bool cluster = s.size >= SC_CL_MIN && (s.size >> rounds) >= (u64)SC_CL;
+    if (!cluster && s.size >= SC_CL_MIN) return 1;
+    ScClusterArgs a{};
     a.a_base = s.a_base;
     for (int c = 0; c < 3; ++c) { a.a[c] = s.a_in[c]; a.b[c] = s.b[c]; }
-    a.size = s.size;
+    a.size = (u32)s.size;
     a.rounds = rounds;
     a.r_slot = s.r_slot;
     a.fold_after = fold_after;
     a.tx = s.tx;
     a.sc = s.sc;
     a.ext2 = s.ext2;
-    // As many warps as round 0 has pairs for (one warp up to 32 pairs): the
-    // rounds are chains of transcript steps, and barriers and cross-warp sums
-    // over idle warps only lengthen them.
-    u32 threads = 32;
-    while (threads < (u32)SC_SMALL_THREADS && threads < (s.size >> 1)) threads <<= 1;
-    k_sumcheck_small<<<1, threads, 0, st>>>(a);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(cluster ? SC_CL : 1);
+    cfg.blockDim = dim3(SC_CL_THREADS + 32);
+    cfg.dynamicSmemBytes = s.size / (cluster ? SC_CL : 1) * 48;
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = SC_CL;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = cluster ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, cluster ? k_sumcheck_cluster<SC_CL> : k_sumcheck_cluster<1>, a) != cudaSuccess) return -1;
     count_launches(1);
     return 0;
 }
@@ -461,7 +550,7 @@ int sumcheck_prepare() {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fns[k], SC_THREADS, 0) != cudaSuccess) return -1;
         g_sc_occ[k] = occ < 1 ? 1 : occ;
     }
-    return device_sms() ? 0 : -1;
+    return device_sms() ? sumcheck_cluster_prepare() : -1;
 }
 
 int launch_sumcheck_round(const SumcheckArgs& s, cudaStream_t st) {

@@ -273,7 +273,7 @@ struct SumcheckArgs {
 // fold fused in.  PoW (if any) and the challenge squeeze happen in-stream.
 int launch_sumcheck_round(const SumcheckArgs& a, cudaStream_t st);
 // All `rounds` rounds of a small sumcheck (and the fold after the last one when
-// fold_after) in one single-CTA kernel: round t's challenge goes to
+// fold_after) in one launch (a cluster): round t's challenge goes to
 // sc_r[r_slot + t].  Returns 1 (nothing launched) when the sumcheck is too
 // large or has round PoW.
 int launch_sumcheck_small(const SumcheckArgs& a, int rounds, int fold_after, cudaStream_t st);

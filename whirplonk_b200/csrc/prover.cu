@@ -257,7 +257,7 @@ int commit_vectors(const Ctx& c, int ci, const uint64_t* const src[3], uint32_t 
 // vector is still the base-field coefficient array (first sumcheck only).
 // Leaves a, cov folded to size >> rounds when `fold_after` is set.
 int sumcheck(const Ctx& c, const SumcheckSchedule& s, uint64_t size, bool base_first, int& r_slot, bool fold_after) {
-    if (s.num_rounds > 0) {  // small sumchecks: one single-CTA kernel for every round
+    if (s.num_rounds > 0) {  // small sumchecks: one launch for every round
         SumcheckArgs a{};
         a.a_base = base_first ? c.w(c.p.off_coeffs) : nullptr;
         for (int k = 0; k < 3; ++k) { a.a_in[k] = c.a(k); a.a_out[k] = c.a(k); a.b[k] = c.cov(k); }
