@@ -616,18 +616,14 @@ __global__ void k_ood_tables(const E3* pts, int n_ood, u32 hi_count, E3* tab, bo
     }
 }
 
-// Sum over coefficients off .. off + len - 1 of chunk h (2^LO coefficients)
-// of vector v against point table j, one value per lane (unreduced products,
-// reduced once, scaled by z_j^(h 2^LO)).  Every load of a batch -- the
+// Sum over coefficients base .. base + len - 1 of vector v against a table of
+// the powers zl[0 ..], one value per lane (unreduced products, reduced once).  Every load of a batch -- the
 // coefficients and their table powers, 4 Ext3 or 8 base elements per lane --
 // is issued before its products, so a warp waits for memory once per batch.
-__device__ __forceinline__ E3 ood_part(const OodArgs& a, const E3* zlo, const E3* zhi, u32 v, u64 h, u32 off,
-                                       u32 len, u32 lane) {
+__device__ __forceinline__ E3 ood_sum(const OodArgs& a, const E3* zl, u32 v, u64 base, u32 len, u32 lane) {
     const u64* b0 = a.v[0] + (u64)v * a.vec_stride;
-    const u64 base = (h << OOD_LO) + off;
     const u64 rest = a.size > base ? a.size - base : 0;
     const u32 cnt = (u32)(rest < len ? rest : len);
-    const E3* zl = zlo + off;
     E3Acc s = e3acc_zero();
     u32 l = lane;
     if (a.ext3) {  // one vector (nvec == 1): components in v[0..2]
@@ -659,7 +655,103 @@ __device__ __forceinline__ E3 ood_part(const OodArgs& a, const E3* zlo, const E3
         }
         for (; l < cnt; l += 32) e3acc_mac_base(s, zl[l], b0[base + l]);
     }
-    return ef_mul(ef_fix(e3acc_reduce(s), a.ext2), zhi[h], a.ext2);
+    return ef_fix(e3acc_reduce(s), a.ext2);
+}
+// The part of chunk h (2^LO coefficients) from off on, scaled by z_j^(h 2^LO).
+__device__ __forceinline__ E3 ood_part(const OodArgs& a, const E3* zlo, const E3* zhi, u32 v, u64 h, u32 off,
+                                       u32 len, u32 lane) {
+    return ef_mul(ood_sum(a, zlo + off, v, (h << OOD_LO) + off, len, lane), zhi[h], a.ext2);
+}
+
+// One value (one vector at one point), in one launch.  Every CTA builds the
+// powers that it needs: z^l for l < len by doubling, beside the chain of
+// squarings z^(2^i) on warp 0.  Warp w takes the parts (len coefficients each)
+// w, w + W, ... from the last one down, acc = acc z^(W len) + part, and scales
+// by z^(w len) at the end; both factors are products of the squarings, a lane a
+// bit.  Bound at small sizes by the chain of squarings and sums, at large ones by
+// the products.  Against a launch of its own for the tables (serial powers, up to
+// two products a bit) and every table entry read through L2, all values of a proof
+// on B200: n = 12 64 -> 47 us (3), n = 16 88 -> 68 (4), n = 18 94 -> 73 (4),
+// n = 20 127 -> 123 (5), n = 24 262 -> 238 (6).  Several values keep the table
+// launch: their powers are shared.
+__global__ void __launch_bounds__(OOD_THREADS) k_ood_one(const __grid_constant__ OodArgs a, u32 len_log, u64 parts,
+                                                         u32 squares, E3* partials, unsigned* counter) {
+    __shared__ E3 zl[1u << OOD_LO];
+    __shared__ E3 pw[64];  // z^(2^i)
+    __shared__ E3 red[32];
+    __shared__ bool is_last;
+    const u32 lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = OOD_THREADS / 32;
+    const bool x2 = a.ext2;
+    const E3 z = a.pts[0];
+    E3 sq = z;
+    if (threadIdx.x == 0) {
+        zl[0] = e3_one();
+        pw[0] = z;
+    }
+    __syncthreads();
+    for (u32 i = 0; i < len_log; ++i) {
+        if (warp == 0) {
+            sq = ef_mul(sq, sq, x2);
+            if (lane == 0) pw[i + 1] = sq;
+        } else {
+            const E3 f = pw[i];
+            for (u32 t = threadIdx.x - 32; t < (1u << i); t += OOD_THREADS - 32) zl[(1u << i) + t] = ef_mul(zl[t], f, x2);
+        }
+        __syncthreads();
+    }
+    if (warp == 0)
+        for (u32 i = len_log + 1; i < squares; ++i) {
+            sq = ef_mul(sq, sq, x2);
+            if (lane == 0) pw[i] = sq;
+        }
+    const u64 gw = (u64)blockIdx.x * nwarps + warp, W = (u64)gridDim.x * nwarps;
+    const u64 count = gw < parts ? (parts - gw + W - 1) / W : 0;
+    E3 acc = e3_zero(), last = e3_zero();
+    if (count) last = ood_sum(a, zl, 0, (gw + (count - 1) * W) << len_log, 1u << len_log, lane);
+    __syncthreads();
+    if (count) {
+        // lanes 0..15: the bits of w; lanes 16..31: the bits of W
+        const u32 b = lane & 15;
+        const u64 e = lane < 16 ? gw : (parts > W ? W : 0);
+        E3 f = ((e >> b) & 1) ? pw[len_log + b] : e3_one();
+#pragma unroll 1
+        for (int o = 8; o > 0; o >>= 1)
+            f = ef_mul(f, E3{__shfl_xor_sync(0xFFFFFFFFu, f.c0, o), __shfl_xor_sync(0xFFFFFFFFu, f.c1, o),
+                             __shfl_xor_sync(0xFFFFFFFFu, f.c2, o)}, x2);
+        const E3 fw{__shfl_sync(0xFFFFFFFFu, f.c0, 0), __shfl_sync(0xFFFFFFFFu, f.c1, 0), __shfl_sync(0xFFFFFFFFu, f.c2, 0)};
+        const E3 fs{__shfl_sync(0xFFFFFFFFu, f.c0, 16), __shfl_sync(0xFFFFFFFFu, f.c1, 16), __shfl_sync(0xFFFFFFFFu, f.c2, 16)};
+        acc = last;
+        for (u64 k = count - 1; k-- > 0;)
+            acc = e3_add(ef_mul(acc, fs, x2), ood_sum(a, zl, 0, (gw + k * W) << len_log, 1u << len_log, lane));
+        acc = ef_mul(acc, fw, x2);
+    }
+    const E3 bs = block_sum_e3(acc, red);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = bs;
+        __threadfence();
+        is_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    E3 tot = e3_zero();
+    for (u32 c = threadIdx.x; c < gridDim.x; c += OOD_THREADS) {
+        const E3* pp = &partials[c];
+        tot = e3_add(tot, E3{__ldcg(&pp->c0), __ldcg(&pp->c1), __ldcg(&pp->c2)});
+    }
+    tot = block_sum_e3(tot, red);
+    if (threadIdx.x == 0) {
+        a.out[0] = tot;
+        red[0] = tot;
+        *counter = 0;
+    }
+    __syncwarp();
+    if (warp == 0) {
+        WarpTx t;
+        wtx_load(t, a.tx);
+        wtx_message_t(t, red[0]);
+        wtx_store(t, a.tx);
+    }
 }
 
 // ITEMS: one warp per (value, chunk) item, partials[k * hi_count + h] (few
@@ -755,15 +847,29 @@ int launch_ood(const OodArgs& a, cudaStream_t st) {
     unsigned* counter = reinterpret_cast<unsigned*>(base);
     E3* partials = reinterpret_cast<E3*>(base + 256);
     E3* tab = partials + (size_t)OOD_GRID * a.scratch_values;
+    const u64 warps_per_cta = OOD_THREADS / 32;
+    const u64 cap = std::min<u64>(4ull * device_sms(), (u64)OOD_GRID);
+    if (a.n_ood == 1 && a.nvec == 1 && a.skip_lo >= a.skip_hi) {
+        // Parts of 2^10 coefficients, of fewer (down to 2^7) while they still fit
+        // the grid's warps once.
+        u32 len_log = OOD_LO;
+        while (len_log > OOD_LO - 3 && (a.size >> (len_log - 1)) <= cap * warps_per_cta) --len_log;
+        const u64 parts = (a.size + (1ull << len_log) - 1) >> len_log;
+        const u64 grid = std::min<u64>(cap, (parts + warps_per_cta - 1) / warps_per_cta);
+        const u64 top = parts > grid * warps_per_cta ? grid * warps_per_cta : parts - 1;  // the largest factor's exponent / len
+        u32 bits = 0;
+        while (top >> bits) ++bits;
+        k_ood_one<<<(unsigned)grid, OOD_THREADS, 0, st>>>(a, len_log, parts, len_log + bits, partials, counter);
+        count_launches(1);
+        return 0;
+    }
     const u64 entries = (u64)((1u << OOD_LO) + hc) * a.n_ood;
     k_ood_tables<<<(unsigned)std::min<u64>(2ull * device_sms(), (entries + 255) / 256), 256, 0, st>>>(a.pts, a.n_ood, hc, tab, a.ext2 != 0);
     count_launches(1);
-    const u64 warps_per_cta = OOD_THREADS / 32;
     const u64 items = (u64)a.n_ood * a.nvec * hc;
     // Few chunks per value: spread (value, chunk) items over the warps (the
     // partials fit: items <= OOD_GRID * scratch_values when hc <= OOD_GRID).
     const bool by_items = hc <= OOD_GRID && items > hc;
-    const u64 cap = std::min<u64>(4ull * device_sms(), (u64)OOD_GRID);
     // Chunks of one value cut into up to 8 parts while the parts still fit
     // the grid's warps once (a part is one product by the chunk's power more).
     u32 sub_log = 0;
