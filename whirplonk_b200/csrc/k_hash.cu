@@ -750,6 +750,7 @@ __global__ void __launch_bounds__(OOD_THREADS) k_ood_one(const __grid_constant__
         WarpTx t;
         wtx_load(t, a.tx);
         wtx_message_t(t, red[0]);
+        if (a.pow_sc) wtx_pow_challenge(t, a.pow_sc);
         wtx_store(t, a.tx);
     }
 }
@@ -827,6 +828,7 @@ __global__ void __launch_bounds__(OOD_THREADS) k_ood(OodArgs a, const E3* tab, u
             const u32 v = k % a.nvec;
             if (v < a.skip_lo || v >= a.skip_hi) wtx_message_t(t, totals[k]);
         }
+        if (a.pow_sc) wtx_pow_challenge(t, a.pow_sc);
         wtx_store(t, a.tx);
     }
     if (threadIdx.x == 0) *counter = 0;

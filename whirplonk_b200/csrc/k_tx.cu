@@ -100,12 +100,8 @@ __global__ void k_pow_challenge(TxState* tx, ProofScalars* sc) {
     if (threadIdx.x >= 32) return;
     WarpTx t;
     wtx_load(t, tx);
-    wtx_squeeze_bytes(t, sc->pow_ch, 32);
+    wtx_pow_challenge(t, sc);
     wtx_store(t, tx);
-    if (threadIdx.x == 0) {
-        sc->pow_best = ~0ull;
-        sc->pow_next = 0;
-    }
 }
 
 // H: 0 = BLAKE3, 1 = SHA-256 (the PoW engine follows the hash_id, whir.hpp:134-140).
@@ -180,32 +176,36 @@ __global__ void k_pow_finish(TxState* tx, ProofScalars* sc, int slot) {
     wtx_store(t, tx);
 }
 
-int launch_pow_search(TxState* tx, ProofScalars* sc, u64 threshold, int hash, cudaStream_t st) {
+int launch_pow_search(TxState* tx, ProofScalars* sc, u64 threshold, int hash, bool drawn, cudaStream_t st) {
     if (threshold == ~0ull) return 0;  // zero difficulty: nothing sent (proof_of_work.hpp:241)
-    k_pow_challenge<<<1, 32, 0, st>>>(tx, sc);
-    count_launches(1);
+    if (!drawn) {
+        k_pow_challenge<<<1, 32, 0, st>>>(tx, sc);
+        count_launches(1);
+    }
     return launch_pow_grind_only(sc, threshold, hash, st);
 }
 int launch_pow(TxState* tx, ProofScalars* sc, u64 threshold, int slot, int hash, cudaStream_t st) {
     if (threshold == ~0ull) return 0;
-    launch_pow_search(tx, sc, threshold, hash, st);
+    launch_pow_search(tx, sc, threshold, hash, false, st);
     k_pow_finish<<<1, 32, 0, st>>>(tx, sc, slot);
     count_launches(1);
     return 0;
 }
 
 // Final vector: prover_message of every coefficient (whir_prover.hpp:360-362).
-// One warp.
-__global__ void k_send_vector(TxState* tx, const u64* c0, const u64* c1, const u64* c2, u64 size) {
+// One warp; pow_sc: the challenge of the PoW that follows, too.
+__global__ void k_send_vector(TxState* tx, const u64* c0, const u64* c1, const u64* c2, u64 size, ProofScalars* pow_sc) {
     if (threadIdx.x >= 32) return;
     WarpTx t;
     wtx_load(t, tx);
     for (u64 i = 0; i < size; ++i) wtx_message_t(t, E3{c0[i], c1[i], c2[i]});
+    if (pow_sc) wtx_pow_challenge(t, pow_sc);
     wtx_store(t, tx);
 }
 
-int launch_send_vector(TxState* tx, const u64* c0, const u64* c1, const u64* c2, u64 size, cudaStream_t st) {
-    k_send_vector<<<1, 32, 0, st>>>(tx, c0, c1, c2, size);
+int launch_send_vector(TxState* tx, const u64* c0, const u64* c1, const u64* c2, u64 size, ProofScalars* pow_sc,
+                       cudaStream_t st) {
+    k_send_vector<<<1, 32, 0, st>>>(tx, c0, c1, c2, size, pow_sc);
     count_launches(1);
     return 0;
 }

@@ -163,6 +163,7 @@ struct OodArgs {
     E3* out;
     u32 out_stride;
     TxState* tx;
+    ProofScalars* pow_sc;     // not null: the PoW challenge that follows the values is drawn, too
     void* scratch;
     u32 scratch_values;       // n_ood * nvec capacity of the scratch
     int ext2;                 // target field GoldilocksExt2 (vectors and points (c0, c1, 0))
@@ -180,12 +181,15 @@ int launch_tx_init(TxState* tx, const unsigned char* ds, u32 ds_len, unsigned ch
 int launch_constraint_rlc(TxState* tx, ProofScalars* sc, int n_forms, int nwit, int ood, int nvec, cudaStream_t st);
 // PoW: squeeze the 32-byte challenge, grind the minimum nonce, send it.
 int launch_pow(TxState* tx, ProofScalars* sc, u64 threshold, int slot, int hash, cudaStream_t st);
-// The challenge and the search; the nonce (sc->pow_best) is sent by k_open.
-int launch_pow_search(TxState* tx, ProofScalars* sc, u64 threshold, int hash, cudaStream_t st);
+// The challenge (unless the kernel before has drawn it) and the search; the nonce
+// (sc->pow_best) is sent by k_open.
+int launch_pow_search(TxState* tx, ProofScalars* sc, u64 threshold, int hash, bool drawn, cudaStream_t st);
 // `count` Ext3 challenges into sc->sc_r[slot ..] (verifier_message_vec).
 int launch_squeeze_challenges(TxState* tx, ProofScalars* sc, int slot, int count, cudaStream_t st);
-// Sends every coefficient of the final folded vector (whir_prover.hpp:360-362).
-int launch_send_vector(TxState* tx, const u64* c0, const u64* c1, const u64* c2, u64 size, cudaStream_t st);
+// Sends every coefficient of the final folded vector (whir_prover.hpp:360-362);
+// pow_sc != null: draws the challenge of the PoW that follows.
+int launch_send_vector(TxState* tx, const u64* c0, const u64* c1, const u64* c2, u64 size, ProofScalars* pow_sc,
+                       cudaStream_t st);
 
 // ---- Opening ------------------------------------------------------------------
 struct OpenArgs {

@@ -213,8 +213,9 @@ struct Ctx {
 // RS encode + leaves + Merkle of commitment `ci` whose message is `vectors`
 // vectors (src planes, vsize words each, consecutive), then the OOD values of
 // those vectors at the commitment's points, stored at out[j * out_stride + v].
+// pow_sc != null: the values' kernel (n_ood > 0) draws the PoW challenge that follows.
 int commit_vectors(const Ctx& c, int ci, const uint64_t* const src[3], uint32_t ncomp, uint64_t vsize,
-                   uint32_t vectors, int n_ood, E3* out, uint32_t out_stride) {
+                   uint32_t vectors, int n_ood, E3* out, uint32_t out_stride, ProofScalars* pow_sc = nullptr) {
     const CommitBuffers& cb = c.p.commits[ci];
     const uint32_t fold_depth = cb.depth / vectors;
     LdeArgs L{};
@@ -247,6 +248,7 @@ int commit_vectors(const Ctx& c, int ci, const uint64_t* const src[3], uint32_t 
     o.out = out;
     o.out_stride = out_stride;
     o.tx = c.tx();
+    o.pow_sc = pow_sc;
     o.scratch = c.ws + c.p.off_ood_scratch;
     o.scratch_values = c.p.ood_values;
     WG_TIMED(c, FAM_OOD, launch_ood(o, c.st));
@@ -434,9 +436,11 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
         // base-field rounds commit the c0 plane only, Ext2 rounds c0 and c1 (c2 is zero)
         const uint32_t deg = (uint32_t)p.params.field_degree;
         const uint64_t* src[3] = {c.a(0), deg >= 2 ? c.a(1) : nullptr, deg >= 2 ? c.a(2) : nullptr};
-        WG_TRY(commit_vectors(c, ci, src, deg, vsize, 1, (int)rc.irs.out_domain, &c.sc()->ood_vals[ci][0], 1));
+        const bool drawn = rc.irs.out_domain > 0 && rc.pow_threshold != ~0ull;
+        WG_TRY(commit_vectors(c, ci, src, deg, vsize, 1, (int)rc.irs.out_domain, &c.sc()->ood_vals[ci][0], 1,
+                              drawn ? c.sc() : nullptr));
         // (the opening sends the nonce)
-        WG_TIMED(c, FAM_POW, launch_pow_search(c.tx(), c.sc(), rc.pow_threshold, c.p.params.hash, st));
+        WG_TIMED(c, FAM_POW, launch_pow_search(c.tx(), c.sc(), rc.pow_threshold, c.p.params.hash, drawn, st));
         // open the previous commitment (the first round: every initial commitment)
         const IrsSchedule& prev = r == 0 ? s.initial : s.rounds[r - 1].irs;
         const CommitBuffers& pb = p.commits[r == 0 ? 0 : ci - 1];
@@ -481,8 +485,9 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
     }
 
     // final vector, PoW, opening, sumcheck
-    WG_TIMED(c, FAM_TX, launch_send_vector(c.tx(), c.a(0), c.a(1), c.a(2), vsize, st));
-    WG_TIMED(c, FAM_POW, launch_pow_search(c.tx(), c.sc(), s.final_pow, c.p.params.hash, st));
+    WG_TIMED(c, FAM_TX, launch_send_vector(c.tx(), c.a(0), c.a(1), c.a(2), vsize,
+                                           s.final_pow != ~0ull ? c.sc() : nullptr, st));
+    WG_TIMED(c, FAM_POW, launch_pow_search(c.tx(), c.sc(), s.final_pow, c.p.params.hash, true, st));
     {
         const bool initial = s.rounds.empty();
         const IrsSchedule& last = initial ? s.initial : s.rounds.back().irs;

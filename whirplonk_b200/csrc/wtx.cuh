@@ -13,6 +13,7 @@
 // same arguments.  A kernel loads the state with wtx_load, runs its steps and
 // writes it back with wtx_store.
 #pragma once
+#include "state.cuh"
 #include "transcript.cuh"
 
 namespace wg {
@@ -333,6 +334,15 @@ __device__ __forceinline__ void wtx_absorb2_t(WarpTx& t, const E3& x, const E3& 
     const bool d1 = t.deg == 1, d2 = t.deg == 2;
     const u64 w[6] = {x.c0, d1 ? y.c0 : x.c1, d2 ? y.c0 : x.c2, d2 ? y.c1 : y.c0, y.c1, y.c2};
     wtx_absorb_words(t, w, 2 * t.deg);
+}
+
+// A PoW's challenge (proof_of_work.hpp), and the search's state reset.
+__device__ __forceinline__ void wtx_pow_challenge(WarpTx& t, ProofScalars* sc) {
+    wtx_squeeze_bytes(t, sc->pow_ch, 32);
+    if (wtx_lane() == 0) {
+        sc->pow_best = ~0ull;
+        sc->pow_next = 0;
+    }
 }
 
 // geometric_challenge (geometric_challenge.hpp:39-44): [] / [1] / squeeze x ->
