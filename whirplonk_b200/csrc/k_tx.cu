@@ -263,15 +263,18 @@ int launch_squeeze_challenges(TxState* tx, ProofScalars* sc, int slot, int count
 // ---------------------------------------------------------------------------
 constexpr int OPEN_THREADS = 512, OPEN_WARPS = OPEN_THREADS / 32;
 constexpr int OPEN_GATHER = OPEN_THREADS - 32;  // threads of the gathering warps
+constexpr int OPEN_SORT = 256;                  // of these, threads that sort while the others take the rows' values
+constexpr u32 OPEN_ROW_WARPS = (OPEN_GATHER - OPEN_SORT) / 32;
 constexpr u32 OPEN_CTAS = 8, OPEN_MAX_LOGN = 26;
 
-// Barrier of the gathering warps, and the same counting `v`.
+// Barriers of the gathering and of the sorting warps, and the latter counting `v`.
 __device__ __forceinline__ void gather_sync() { asm volatile("bar.sync 1, %0;" ::"n"(OPEN_GATHER) : "memory"); }
-__device__ __forceinline__ u32 gather_count(bool v) {
+__device__ __forceinline__ void sort_sync() { asm volatile("bar.sync 2, %0;" ::"n"(OPEN_SORT) : "memory"); }
+__device__ __forceinline__ u32 sort_count(bool v) {
     u32 r;
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.popc.u32 %0, 1, %2, p;\n\t}"
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.popc.u32 %0, 2, %2, p;\n\t}"
                  : "=r"(r)
-                 : "r"((u32)v), "n"(OPEN_GATHER)
+                 : "r"((u32)v), "n"(OPEN_SORT)
                  : "memory");
     return r;
 }
@@ -285,6 +288,8 @@ __global__ void __launch_bounds__(OPEN_THREADS) k_open(OpenArgs a) {
     __shared__ u32 cnt[OPEN_MAX_LOGN][MAX_QUERIES / 32];  // emitted siblings per level and chunk of 32 nodes, then their prefix
     __shared__ u32 lvl[OPEN_MAX_LOGN + 1];                // siblings of the levels below, and of all
     __shared__ E3 red[OPEN_WARPS];
+    __shared__ u64 gpow[32];  // gen^(2^i)
+    __shared__ u32 distinct;
     __shared__ bool last;
     const TxState* tx = a.tx;  // the hint stream (unchanged until the last CTA's store)
     ProofScalars* sc = a.sc;
@@ -317,6 +322,10 @@ __global__ void __launch_bounds__(OPEN_THREADS) k_open(OpenArgs a) {
             }
             eqw[i] = acc;
         }
+        if (t == OPEN_THREADS - 1) {
+            u64 p = a.gen;
+            for (u32 i = 0; i < a.logN; ++i, p = gl_mul(p, p)) gpow[i] = p;
+        }
     }
     __syncthreads();
     u64 blk = 0;  // hint bytes of one commitment (gathering warps)
@@ -336,13 +345,88 @@ __global__ void __launch_bounds__(OPEN_THREADS) k_open(OpenArgs a) {
         }
         gather_sync();
 
-        // 3. STIR point and value of each opened row: a warp per row, its lanes
-        //    over the row's elements (all commitments side by side), a warp sum.
-        if (a.stir) {
+        u32 u = 0;  // distinct indices
+        // Merkle levels.  Per level L the nodes are the distinct values x of
+        // cur[j] >> L (cur is sorted, so equal values are adjacent); x emits its
+        // sibling x ^ 1 unless the sibling is itself a node, i.e. the
+        // neighbouring distinct value: an odd x decides at its first j, an even
+        // x at its last.  Siblings are emitted level by level, increasing x
+        // within a level.
+        auto emits = [&](u32 j, u32 L) -> bool {
+            if (j >= u) return false;
+            const u64 x = cur[j] >> L;
+            if (x & 1) {
+                if (j == 0) return true;
+                const u64 p = cur[j - 1] >> L;
+                return p != x && p != x - 1;
+            }
+            if (j + 1 == u) return true;
+            const u64 n = cur[j + 1] >> L;
+            return n != x && n != x + 1;
+        };
+        auto exclusive = [&](u32 v, u32& total) {
+            u32 incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const u32 w = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= (u32)o) incl += w;
+            }
+            total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            return incl - v;
+        };
+        if (warp <= OPEN_SORT / 32) {
+            // Sort + dedup: a value goes to slot #{distinct values below it}.  Two
+            // lanes share an index's comparisons.
+            for (u32 i0 = 0; i0 < q; i0 += OPEN_SORT / 2) {
+                const u32 i = i0 + (g >> 1);
+                const u64 v = i < q ? idx_s[i] : 0;
+                bool d = false;
+                for (u32 j = g & 1; j < i && i < q; j += 2) d |= idx_s[j] == v;
+                d |= __shfl_xor_sync(0xFFFFFFFFu, (int)d, 1);
+                if (i < q) dup[i] = d;
+                u += sort_count(i < q && !d && (g & 1) == 0);
+            }
+            for (u32 i0 = 0; i0 < q; i0 += OPEN_SORT / 2) {
+                const u32 i = i0 + (g >> 1);
+                const u64 v = i < q ? idx_s[i] : 0;
+                u32 lt = 0;
+                for (u32 j = g & 1; j < q; j += 2) lt += idx_s[j] < v && !dup[j];
+                lt += __shfl_xor_sync(0xFFFFFFFFu, lt, 1);
+                if (i < q && !dup[i] && (g & 1) == 0) cur[lt] = v;
+            }
+            sort_sync();
+
+            const u32 chunks = (u + 31) / 32;
+            for (u32 it = warp - 1; it < a.logN * chunks; it += OPEN_SORT / 32) {
+                const u32 L = it / chunks, c = it % chunks;
+                const u32 m = __popc(__ballot_sync(0xFFFFFFFFu, emits(c * 32 + lane, L)));
+                if (lane == 0) cnt[L][c] = m;
+            }
+            sort_sync();
+            for (u32 L = warp - 1; L < a.logN; L += OPEN_SORT / 32) {
+                u32 total;
+                const u32 e = exclusive(lane < chunks ? cnt[L][lane] : 0, total);
+                if (lane < chunks) cnt[L][lane] = e;
+                if (lane == 0) lvl[L] = total;
+            }
+            sort_sync();
+            if (warp == 1) {
+                u32 total;
+                const u32 e = exclusive(lane < a.logN ? lvl[lane] : 0, total);
+                if (lane <= a.logN) lvl[lane] = e;
+            }
+            if (g == 0) distinct = u;
+        } else if (a.stir) {
+            // 3. STIR point and value of each opened row: a warp per row, its lanes
+            //    over the row's elements (all commitments side by side), a warp sum.
             const u32 dmask = (1u << a.fold) - 1;
             const u32 elems = nwit * a.depth;
-            for (u32 i = ggw; i < q; i += ggws) {
+            const u32 rows = gridDim.x * OPEN_ROW_WARPS;
+            for (u32 i = blockIdx.x * OPEN_ROW_WARPS + warp - 1 - OPEN_SORT / 32; i < q; i += rows) {
                 const u64 id = codeword_row(idx_s[i], a.logN, a.perm_log_e);  // natural row = exponent of its point
+                u64 pt = lane < a.logN && ((id >> lane) & 1) ? gpow[lane] : 1;  // gen^id, a lane a bit
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) pt = gl_mul(pt, __shfl_xor_sync(0xFFFFFFFFu, pt, o));
                 E3 val = e3_zero();
                 for (u32 k = lane; k < elems; k += 32) {
                     const u32 w = k / a.depth, el = k - w * a.depth;
@@ -363,82 +447,14 @@ __global__ void __launch_bounds__(OPEN_THREADS) k_open(OpenArgs a) {
                 }
                 val = e3_warp_sum(val);
                 if (lane == 0) {
-                    sc->stir_pts[a.ood_offset + i] = e3_base(gl_pow(a.gen, id));
+                    sc->stir_pts[a.ood_offset + i] = e3_base(pt);
                     sc->stir_vals[a.ood_offset + i] = val;
                 }
             }
         }
-
-        // Sort + dedup: a value goes to slot #{distinct values below it}.  Two
-        // lanes share an index's comparisons.
-        u32 u = 0;
-        for (u32 i0 = 0; i0 < q; i0 += OPEN_GATHER / 2) {
-            const u32 i = i0 + (g >> 1);
-            const u64 v = i < q ? idx_s[i] : 0;
-            bool d = false;
-            for (u32 j = g & 1; j < i && i < q; j += 2) d |= idx_s[j] == v;
-            d |= __shfl_xor_sync(0xFFFFFFFFu, (int)d, 1);
-            if (i < q) dup[i] = d;
-            u += gather_count(i < q && !d && (g & 1) == 0);
-        }
-        for (u32 i0 = 0; i0 < q; i0 += OPEN_GATHER / 2) {
-            const u32 i = i0 + (g >> 1);
-            const u64 v = i < q ? idx_s[i] : 0;
-            u32 lt = 0;
-            for (u32 j = g & 1; j < q; j += 2) lt += idx_s[j] < v && !dup[j];
-            lt += __shfl_xor_sync(0xFFFFFFFFu, lt, 1);
-            if (i < q && !dup[i] && (g & 1) == 0) cur[lt] = v;
-        }
         gather_sync();
-
-        // Merkle levels.  Per level L the nodes are the distinct values x of
-        // cur[j] >> L (cur is sorted, so equal values are adjacent); x emits its
-        // sibling x ^ 1 unless the sibling is itself a node, i.e. the
-        // neighbouring distinct value: an odd x decides at its first j, an even
-        // x at its last.  Siblings are emitted level by level, increasing x
-        // within a level.
+        u = distinct;
         const u32 nchunk = (u + 31) / 32;
-        auto emits = [&](u32 j, u32 L) -> bool {
-            if (j >= u) return false;
-            const u64 x = cur[j] >> L;
-            if (x & 1) {
-                if (j == 0) return true;
-                const u64 p = cur[j - 1] >> L;
-                return p != x && p != x - 1;
-            }
-            if (j + 1 == u) return true;
-            const u64 n = cur[j + 1] >> L;
-            return n != x && n != x + 1;
-        };
-        for (u32 it = warp - 1; it < a.logN * nchunk; it += OPEN_WARPS - 1) {
-            const u32 L = it / nchunk, c = it % nchunk;
-            const u32 m = __popc(__ballot_sync(0xFFFFFFFFu, emits(c * 32 + lane, L)));
-            if (lane == 0) cnt[L][c] = m;
-        }
-        gather_sync();
-        auto exclusive = [&](u32 v, u32& total) {
-            u32 incl = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const u32 w = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-                if (lane >= (u32)o) incl += w;
-            }
-            total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            return incl - v;
-        };
-        for (u32 L = warp - 1; L < a.logN; L += OPEN_WARPS - 1) {
-            u32 total;
-            const u32 e = exclusive(lane < nchunk ? cnt[L][lane] : 0, total);
-            if (lane < nchunk) cnt[L][lane] = e;
-            if (lane == 0) lvl[L] = total;
-        }
-        gather_sync();
-        if (warp == 1) {
-            u32 total;
-            const u32 e = exclusive(lane < a.logN ? lvl[lane] : 0, total);
-            if (lane <= a.logN) lvl[lane] = e;
-        }
-        gather_sync();
         const u64 merkle_bytes = 32ull * lvl[a.logN];
         const u64 esz = 8ull * a.ncomp;
         const u64 row_bytes = esz * a.depth;
@@ -547,8 +563,8 @@ int launch_open(const OpenArgs& a, cudaStream_t st) {
     if (a.q > (u32)MAX_QUERIES || (1u << a.fold) > (u32)MAX_DEPTH || a.nwit < 1 || a.nwit > (u32)MAX_WITNESSES) return -1;
     if (a.stir && (a.depth & ((1u << a.fold) - 1)) != 0) return -1;
     if (a.logN > OPEN_MAX_LOGN || a.ood_offset > MAX_OOD) return -1;
-    // A CTA per 15 rows (one row a warp), at most OPEN_CTAS.
-    const u32 rows = OPEN_WARPS - 1, ctas = std::min(OPEN_CTAS, std::max(1u, (a.q + rows - 1) / rows));
+    // A row a warp of those that take the values, at most OPEN_CTAS.
+    const u32 rows = OPEN_ROW_WARPS, ctas = std::min(OPEN_CTAS, std::max(1u, (a.q + rows - 1) / rows));
     k_open<<<ctas, OPEN_THREADS, 0, st>>>(a);
     count_launches(1);
     return 0;

@@ -183,31 +183,6 @@ __device__ __forceinline__ void wtx_reader(WarpTx& t) {
     t.rpos = 0;
     t.has_reader = 1;
 }
-// Next 8 squeezed bytes as a LE word (any alignment); the result is warp-uniform.
-__device__ __forceinline__ u64 wtx_squeeze_word(WarpTx& t) {
-    wtx_reader(t);
-    if ((t.rpos & 7) == 0) {
-        if (t.rpos == TX_RATE) {
-            t.r = keccak_f1600_warp(t.r);
-            t.rpos = 0;
-        }
-        const u64 v = __shfl_sync(0xFFFFFFFFu, t.r, t.rpos >> 3);
-        t.rpos += 8;
-        return v;
-    }
-    u64 v = 0;
-#pragma unroll 1
-    for (int b = 0; b < 8; ++b) {
-        if (t.rpos == TX_RATE) {
-            t.r = keccak_f1600_warp(t.r);
-            t.rpos = 0;
-        }
-        const u64 w = __shfl_sync(0xFFFFFFFFu, t.r, t.rpos >> 3);
-        v |= ((w >> (8 * (t.rpos & 7))) & 0xFF) << (8 * b);
-        ++t.rpos;
-    }
-    return v;
-}
 // n squeezed bytes into dst (shared or global memory), written by the warp.
 __device__ __forceinline__ void wtx_squeeze_bytes(WarpTx& t, u8* dst, unsigned n) {
     if (n == 0) return;
@@ -266,43 +241,39 @@ __device__ __forceinline__ void wtx_message_u64(WarpTx& t, u64 v) {
     wtx_message_words(t, w);
 }
 
-// 40 squeezed bytes as a LE integer mod p (five words folded from the top).
-__device__ __forceinline__ u64 wtx_challenge_base(WarpTx& t) {
-    u64 w[5];
-#pragma unroll
-    for (int i = 0; i < 5; ++i) w[i] = wtx_squeeze_word(t);
-    u64 acc = gl_reduce(w[4], 0);
-    for (int i = 3; i >= 0; --i) acc = gl_reduce(w[i], acc);
-    return acc;
-}
-
-// ncomp (<= 3) consecutive base-field challenges, lane-parallel when their
-// 40 ncomp bytes start word-aligned inside the current reader block: lane c
-// gathers the five words of challenge c and folds them as above.  Otherwise the
-// challenges are squeezed word by word.  Returns challenge c in component c.
+// ncomp (<= 3) consecutive base-field challenges, challenge c in component c:
+// 40 squeezed bytes each as a LE integer mod p (five words folded from the top).
+// Lane c gathers the six state words that hold challenge c at any alignment -- the
+// index bytes of an opening leave the reader between words -- from this block and,
+// past its end, the next.  (Byte by byte an unaligned Ext3 challenge took ~12 k
+// cycles on B200, this ~1 k.)
 __device__ __forceinline__ E3 wtx_challenges(WarpTx& t, u32 ncomp) {
+    constexpr u32 RW = TX_RATE / 8;
     wtx_reader(t);
     const unsigned l = wtx_lane();
-    if ((t.rpos & 7) == 0 && t.rpos + 40 * ncomp <= TX_RATE) {
-        const u32 src = (t.rpos >> 3) + (l < ncomp ? 5 * l : 0);
-        u64 w[5];
+    const u32 end = t.rpos + 40 * ncomp, sh = 8 * (t.rpos & 7);
+    const u32 src = (t.rpos >> 3) + (l < ncomp ? 5 * l : 0);
+    u64 w[6];
 #pragma unroll
-        for (u32 q = 0; q < 5; ++q) w[q] = __shfl_sync(0xFFFFFFFFu, t.r, src + q);
-        u64 s = gl_reduce(w[4], 0);
+    for (u32 q = 0; q < 6; ++q) w[q] = __shfl_sync(0xFFFFFFFFu, t.r, src + q);
+    if (end > TX_RATE) {
+        t.r = keccak_f1600_warp(t.r);
 #pragma unroll
-        for (int q = 3; q >= 0; --q) s = gl_reduce(w[q], s);
-        t.rpos += 40 * ncomp;
-        const u64 c0 = __shfl_sync(0xFFFFFFFFu, s, 0);
-        const u64 c1 = __shfl_sync(0xFFFFFFFFu, s, 1);
-        const u64 c2 = __shfl_sync(0xFFFFFFFFu, s, 2);
-        return E3{c0, ncomp > 1 ? c1 : 0, ncomp > 2 ? c2 : 0};
+        for (u32 q = 0; q < 6; ++q) {
+            const u64 v = __shfl_sync(0xFFFFFFFFu, t.r, src + q - RW);
+            if (src + q >= RW) w[q] = v;
+        }
     }
-    E3 r{0, 0, 0};
-    r.c0 = wtx_challenge_base(t);
-    if (ncomp > 1) r.c1 = wtx_challenge_base(t);
-    if (ncomp > 2) r.c2 = wtx_challenge_base(t);
-    return r;
+    t.rpos = end > TX_RATE ? end - TX_RATE : end;
+    u64 s = 0;
+#pragma unroll
+    for (int q = 4; q >= 0; --q) s = gl_reduce(sh ? (w[q] >> sh) | (w[q + 1] << (64 - sh)) : w[q], s);
+    const u64 c0 = __shfl_sync(0xFFFFFFFFu, s, 0);
+    const u64 c1 = __shfl_sync(0xFFFFFFFFu, s, 1);
+    const u64 c2 = __shfl_sync(0xFFFFFFFFu, s, 2);
+    return E3{c0, ncomp > 1 ? c1 : 0, ncomp > 2 ? c2 : 0};
 }
+__device__ __forceinline__ u64 wtx_challenge_base(WarpTx& t) { return wtx_challenges(t, 1).c0; }
 __device__ __forceinline__ E3 wtx_challenge_e3(WarpTx& t) { return wtx_challenges(t, 3); }
 
 // Elements of the protocol's target field.  With the base field as target
