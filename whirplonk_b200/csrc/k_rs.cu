@@ -102,11 +102,15 @@ LdeArgs lde_args(whirgpu_ctx* c, const u64* src, u64 m, u32 planes, u32 logN, u6
     return L;
 }
 
-// The inter-pass tables of the form launch_lde takes for a shape.
-void prepare_shape_tables(whirgpu_ctx* c, u32 logN, u32 logX, u32 planes) {
+// The inter-pass tables of the form launch_lde takes for a shape: buffers that do
+// not start at 16 bytes run as butterfly passes.
+void prepare_shape_tables(whirgpu_ctx* c, u32 logN, u32 logX, u32 planes, const u64* src, const u64* tmp) {
     std::lock_guard<std::recursive_mutex> lk(c->cache_mu);
     const uint64_t room = c->budget ? (c->budget > c->allocated ? c->budget - c->allocated : 0) : ~0ull;
-    lde_tables_prepare(c->lde_tables, logN, logX, planes, c->tw.tw_hi, c->tw.tw_lo, c->stream, room);
+    if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(tmp)) & 15) == 0)
+        lde_tables_prepare(c->lde_tables, logN, logX, planes, c->tw.tw_hi, c->tw.tw_lo, c->stream, room);
+    else
+        lde_tables_prepare_plan(c->lde_tables, plan_lde(logN, logX), c->tw.tw_hi, c->tw.tw_lo, c->stream, room);
 }
 
 // The inter-pass tables of `pl` (kernel-level calls run outside graph capture).
@@ -135,7 +139,7 @@ whirgpu_status whirgpu_rs_encode(whirgpu_ctx* c, const uint64_t* d_vectors, size
     const u64 planes = (u64)count << log_depth;
     if (planes > 65535) return fail(c, WHIRGPU_E_INVALID, "too many planes");
     const u32 logN = log_len - log_depth + log_expansion;
-    prepare_shape_tables(c, logN, log_expansion, (u32)planes);
+    prepare_shape_tables(c, logN, log_expansion, (u32)planes, d_vectors, d_tmp);
     const LdeArgs L = lde_args(c, d_vectors, 1ull << (log_len - log_depth), (u32)planes, logN, d_tmp, d_planes);
     if (launch_lde(L, c->stream) != 0) return fail(c, WHIRGPU_E_INVALID, "LDE launch");
     const cudaError_t e = cudaGetLastError();
@@ -151,7 +155,7 @@ whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* c, const uint64_t* vectors, 
     const u32 logN = log_len - log_depth + log_expansion;
     const u64 N = 1ull << logN;
     const u64 in_words = count << log_len;
-    prepare_shape_tables(c, logN, log_expansion, (u32)planes);
+    prepare_shape_tables(c, logN, log_expansion, (u32)planes, location == WHIRGPU_INPUT_DEVICE ? vectors : nullptr, nullptr);
     const u64 node_words = (2 * N) * 8;  // 32-bit words of one tree's node array
     const size_t bytes = (location == WHIRGPU_INPUT_DEVICE ? 0 : in_words * 8) + 2 * planes * N * 8 +
                          count * node_words * 4 + 256;
