@@ -104,7 +104,8 @@ struct TscTabArgs {
     const u64* points;  // n_forms * n * 3 words
     u32 n, k, L, lo_bits, hi_bits;
     int n_forms, n_ood;
-    const ProofScalars* sc;
+    ProofScalars* sc;
+    TxState* tx;
     E3* top;  // [t][B]
     E3* lo;   // [t][l]
     E3* hi;   // [t][h]
@@ -121,26 +122,35 @@ __device__ __forceinline__ E3 eq_range(const u64* pt, u32 c0, u32 bits, u32 v) {
     return r;
 }
 
+// Block 0: the constraint RLC (one warp of transcript steps), beside the tables,
+// which wait for nothing of it -- the terms' coefficients enter in k_tsc_rounds.
+// A launch of its own before the tables (16 us under the profiler, the tables 14):
+// n = 16 on B200 12 us more a proof.
 __global__ void k_tsc_tables(TscTabArgs a) {
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < 32) wtx_constraint_rlc(a.tx, a.sc, a.n_forms, 1, a.n_ood, 1);
+        return;
+    }
     const u32 nt = 1u << a.k, nl = 1u << a.lo_bits, nh = 1u << a.hi_bits;
     const u32 per = nt + nl + nh;
     const int T = a.n_forms + a.n_ood;
     const u64 total = (u64)per * T;
-    for (u64 e = (u64)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (u64)gridDim.x * blockDim.x) {
+    const u64 threads = (u64)(gridDim.x - 1) * blockDim.x;
+    for (u64 e = (u64)(blockIdx.x - 1) * blockDim.x + threadIdx.x; e < total; e += threads) {
         const int t = (int)(e / per);
         const u32 q = (u32)(e % per);
         if (t < a.n_forms) {
             const u64* pt = a.points + (u64)t * a.n * 3;
-            if (q < nt) {  // linear_forms[0] is accumulated with scalar ONE (whir_prover.hpp:161)
-                a.top[(u64)t * nt + q] = e3_mul(t == 0 ? e3_one() : a.sc->crlc[t], eq_range(pt, 0, a.k, q));
+            if (q < nt) {
+                a.top[(u64)t * nt + q] = eq_range(pt, 0, a.k, q);
             } else if (q < nt + nl) {
                 a.lo[(u64)t * nl + (q - nt)] = eq_range(pt, a.n - a.lo_bits, a.lo_bits, q - nt);
             } else {
                 a.hi[(u64)t * nh + (q - nt - nl)] = eq_range(pt, a.k, a.hi_bits, q - nt - nl);
             }
         } else {
-            const E3 z = a.sc->init_ood_pts[t - a.n_forms];
-            if (q < nt) a.top[(u64)t * nt + q] = e3_mul(a.sc->crlc[t], e3_pow(z, (u64)q << a.L));
+            const E3 z = a.sc->ood_pts[0][t - a.n_forms];  // (block 0 writes init_ood_pts)
+            if (q < nt) a.top[(u64)t * nt + q] = e3_pow(z, (u64)q << a.L);
             else if (q < nt + nl) a.lo[(u64)t * nl + (q - nt)] = e3_pow(z, q - nt);
             else a.hi[(u64)t * nh + (q - nt - nl)] = e3_pow(z, (u64)(q - nt - nl) << a.lo_bits);
         }
@@ -221,7 +231,7 @@ __global__ void __launch_bounds__(TSC_SPAN_MAX, 1) k_tsc_eval(TscEvalArgs a) {
 
 struct TscRoundArgs {
     u32 k, parts, hi_bits;
-    int T, r_slot;
+    int T, n_forms, r_slot;
     const E3* part;
     const E3* top;
     E3* hi;   // rescaled in place by the folded G_t
@@ -241,6 +251,8 @@ __global__ void __launch_bounds__(256) k_tsc_rounds(TscRoundArgs a) {
     __shared__ E3 scr[256];
     const u32 nb = 1u << a.k;
     const u32 nv = (u32)a.T * nb;
+    // A term's coefficient; linear_forms[0] is accumulated with scalar ONE (whir_prover.hpp:161).
+    auto term = [&](u32 t) { return t == 0 && a.n_forms > 0 ? e3_one() : a.sc->crlc[t]; };
     if (nv <= blockDim.x && blockDim.x <= 256) {
         // blockDim / nv threads per value, each over a strided share of its
         // partials (independent loads in flight), then one sum per value.
@@ -256,7 +268,7 @@ __global__ void __launch_bounds__(256) k_tsc_rounds(TscRoundArgs a) {
             E3 t = scr[threadIdx.x];
             for (u32 k = 1; k < per; ++k) t = e3_add(t, scr[threadIdx.x + k * nv]);
             Z[threadIdx.x] = t;
-            G[threadIdx.x] = a.top[threadIdx.x];
+            G[threadIdx.x] = e3_mul(term(threadIdx.x / nb), a.top[threadIdx.x]);
         }
     } else {
         for (u32 v = threadIdx.x; v < nv; v += blockDim.x) {
@@ -264,7 +276,7 @@ __global__ void __launch_bounds__(256) k_tsc_rounds(TscRoundArgs a) {
             const E3* p = a.part + (u64)v * a.parts;
             for (u32 q = 0; q < a.parts; ++q) z = e3_add(z, p[q]);
             Z[v] = z;
-            G[v] = a.top[v];
+            G[v] = e3_mul(term(v / nb), a.top[v]);
         }
     }
     __syncthreads();
@@ -276,15 +288,27 @@ __global__ void __launch_bounds__(256) k_tsc_rounds(TscRoundArgs a) {
         E3 sum = sc->sum;
         for (u32 r = 0; r < a.k; ++r) {
             const u32 h = nb >> (r + 1);
-            E3 c0 = e3_zero(), c2 = e3_zero();
-            for (u32 v = lane; v < (u32)a.T * h; v += 32) {
-                const u32 t = v / h, i = v % h;
-                const E3 zl = Z[t * nb + i], zh = Z[t * nb + i + h], gl = G[t * nb + i], gh = G[t * nb + i + h];
-                c0 = e3_add(c0, e3_mul(zl, gl));
-                c2 = e3_add(c2, e3_mul(e3_sub(zh, zl), e3_sub(gh, gl)));
+            // two lanes a pair: the even one sums c0, the odd one c2
+            E3 s = e3_zero();
+            for (u32 v = lane; v < 2 * (u32)a.T * h; v += 32) {
+                const u32 t = (v >> 1) / h, i = (v >> 1) % h;
+                E3 z = Z[t * nb + i], g = G[t * nb + i];
+                if (v & 1) {
+                    z = e3_sub(Z[t * nb + i + h], z);
+                    g = e3_sub(G[t * nb + i + h], g);
+                }
+                s = e3_add(s, e3_mul(z, g));
             }
-            c0 = wtx_sum(c0);
-            c2 = wtx_sum(c2);
+#pragma unroll 1
+            for (int o = 16; o > 1; o >>= 1) {
+                s.c0 = gl_add(s.c0, __shfl_xor_sync(0xFFFFFFFFu, s.c0, o));
+                s.c1 = gl_add(s.c1, __shfl_xor_sync(0xFFFFFFFFu, s.c1, o));
+                s.c2 = gl_add(s.c2, __shfl_xor_sync(0xFFFFFFFFu, s.c2, o));
+            }
+            auto from = [&](int l) {
+                return E3{__shfl_sync(0xFFFFFFFFu, s.c0, l), __shfl_sync(0xFFFFFFFFu, s.c1, l), __shfl_sync(0xFFFFFFFFu, s.c2, l)};
+            };
+            const E3 c0 = from(0), c2 = from(1);
             wtx_absorb2_t(wt, c0, c2);
             const E3 rn = wtx_challenge_t(wt);
             wtx_narg_t(wt, c0);
@@ -386,6 +410,7 @@ int launch_tsc(const TscArgs& s, cudaStream_t st) {
     const u32 sms = device_sms();
     const TscGeom g = tsc_geom(s.n, s.k, sms);
     if (g.parts > tsc_parts_bound(s.n, s.k)) return -1;
+    if (s.n_forms > MAX_FORMS || s.n_ood > MAX_OOD) return -1;
     const TscLayout l = tsc_layout(s.n, s.k, T, g.parts);
     if (l.total > s.scratch_bytes) return -1;
     char* base = reinterpret_cast<char*>(s.scratch);
@@ -395,9 +420,9 @@ int launch_tsc(const TscArgs& s, cudaStream_t st) {
     E3* part = reinterpret_cast<E3*>(base + l.part);
     E3* eqr = reinterpret_cast<E3*>(base + l.eqr);
 
-    TscTabArgs ta{s.points, s.n, s.k, g.L, g.lo_bits, g.hi_bits, s.n_forms, s.n_ood, s.sc, top, lo, hi};
+    TscTabArgs ta{s.points, s.n, s.k, g.L, g.lo_bits, g.hi_bits, s.n_forms, s.n_ood, s.sc, s.tx, top, lo, hi};
     const u64 entries = (u64)T * ((1u << s.k) + (1u << g.lo_bits) + (1u << g.hi_bits));
-    k_tsc_tables<<<(unsigned)std::min<u64>(2ull * sms, (entries + 255) / 256), 256, 0, st>>>(ta);
+    k_tsc_tables<<<1 + (unsigned)std::min<u64>(2ull * sms, (entries + 255) / 256), 256, 0, st>>>(ta);
     count_launches(1);
 
     const unsigned grid = (1u << s.k) * g.chunks * g.cg;
@@ -409,7 +434,7 @@ int launch_tsc(const TscArgs& s, cudaStream_t st) {
         count_launches(1);
     }
 
-    TscRoundArgs ra{s.k, g.parts, g.hi_bits, T, s.r_slot, part, top, hi, eqr, s.tx, s.sc};
+    TscRoundArgs ra{s.k, g.parts, g.hi_bits, T, s.n_forms, s.r_slot, part, top, hi, eqr, s.tx, s.sc};
     k_tsc_rounds<<<1, 256, 0, st>>>(ra);
     count_launches(1);
 

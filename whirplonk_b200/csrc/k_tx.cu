@@ -43,31 +43,8 @@ int launch_tx_init(TxState* tx, const unsigned char* ds, u32 ds_len, unsigned ch
     return 0;
 }
 
-// Vector RLC, constraint RLC and "the sum" (whir_prover.hpp:122-197):
-//   vrlc = geometric_challenge(V), crlc = geometric_challenge(F + O),
-//   sum  = sum_f crlc_f sum_v vrlc_v eval_(f,v) + sum_i crlc_(F+i) sum_v vrlc_v ood_(i,v)
-// over the O = nwit * ood initial OOD points, whose coordinates are also laid
-// out contiguously for the covector.  One warp.
 __global__ void k_constraint_rlc(TxState* tx, ProofScalars* sc, int n_forms, int nwit, int ood, int nvec) {
-    if (threadIdx.x >= 32) return;
-    const int l = threadIdx.x;
-    const int n_ood = nwit * ood;
-    for (int i = l; i < n_ood; i += 32) sc->init_ood_pts[i] = sc->ood_pts[i / ood][i % ood];
-    const int count = n_forms + n_ood;
-    WarpTx t;
-    wtx_load(t, tx);
-    wtx_geometric(t, sc->vrlc, nvec);
-    wtx_geometric(t, sc->crlc, count);
-    wtx_store(t, tx);
-    E3 v = e3_zero();
-    for (int r = l; r < count; r += 32) {
-        const E3* vals = r < n_forms ? &sc->forms_eval[r * nvec] : &sc->init_ood_mat[(r - n_forms) * nvec];
-        E3 row = e3_zero();
-        for (int k = 0; k < nvec; ++k) row = e3_add(row, ef_mul(sc->vrlc[k], vals[k], t.deg == 2));
-        v = e3_add(v, ef_mul(sc->crlc[r], row, t.deg == 2));
-    }
-    v = wtx_sum(v);
-    if (l == 0) sc->sum = v;
+    if (threadIdx.x < 32) wtx_constraint_rlc(tx, sc, n_forms, nwit, ood, nvec);
 }
 
 int launch_constraint_rlc(TxState* tx, ProofScalars* sc, int n_forms, int nwit, int ood, int nvec, cudaStream_t st) {

@@ -285,7 +285,8 @@ int launch_sumcheck_small(const SumcheckArgs& a, int rounds, int fold_after, cud
 int launch_fold(const SumcheckArgs& a, cudaStream_t st);
 size_t sumcheck_scratch_bytes();
 // The initial sumcheck of one base-field vector against a covector of MLE
-// forms and OOD points, by block evaluation (k_sc_tensor.cu): the k rounds'
+// forms and OOD points, by block evaluation (k_sc_tensor.cu): the constraint RLC
+// and the initial sum (as launch_constraint_rlc), the k rounds'
 // messages and challenges (sc_r[r_slot ..]), and the vector and covector folded
 // to size 2^(n - k) in a_out / cov_out -- the state the round kernels reach,
 // without writing the 2^n covector.  Target field Ext3 or the base field.
@@ -293,7 +294,7 @@ struct TscArgs {
     const u64* coeffs;  // 2^n base coefficients
     u32 n, k;           // variables, initial-sumcheck rounds (no round PoW)
     const u64* points;  // n_forms MLE points, n Ext3 coordinates each
-    int n_forms, n_ood; // terms: the forms, then sc->init_ood_pts[0 .. n_ood)
+    int n_forms, n_ood; // terms: the forms, then sc->ood_pts[0][0 .. n_ood)
     ProofScalars* sc;
     TxState* tx;
     int r_slot;

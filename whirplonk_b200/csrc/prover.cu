@@ -360,7 +360,6 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
             WG_TIMED(c, FAM_OOD, launch_ood(o, st));
         }
     }
-    WG_TIMED(c, FAM_TX, launch_constraint_rlc(c.tx(), c.sc(), p.n_forms, (int)W, ood0, (int)V, st));
     const bool has_constraints = p.n_forms + ood0 > 0;
     int r_slot = 0;
     // One base-field vector whose covector is MLE forms and OOD points only:
@@ -370,6 +369,8 @@ int enqueue_prove(const ProofPlan& p, char* ws, const DeviceTables& tw, cudaStre
     const bool tensor = has_constraints && V == 1 && !p.full_vector && p.dense_mask == 0 &&
                         p.params.field_degree != 2 && s.initial_sumcheck.pow_threshold == ~0ull &&
                         tsc_applicable(p.n, k0, p.n_forms + ood0 * (int)W);
+    // (the block evaluation takes the constraint RLC along)
+    if (!tensor) WG_TIMED(c, FAM_TX, launch_constraint_rlc(c.tx(), c.sc(), p.n_forms, (int)W, ood0, (int)V, st));
     if (tensor) {
         TscArgs ta{};
         ta.coeffs = c.w(p.off_coeffs);

@@ -167,9 +167,27 @@ __device__ __forceinline__ void wtx_absorb_words(WarpTx& t, const u64 (&w)[N], u
         wtx_absorb_byte(t, (u8)(v >> (8 * (i & 7))));
     }
 }
+// n bytes from memory, a lane the up to eight bytes of its word (byte by byte over
+// the warp they took ~20 cycles each).
 __device__ __forceinline__ void wtx_absorb_bytes(WarpTx& t, const u8* src, unsigned n) {
     t.has_reader = 0;
-    for (unsigned i = 0; i < n; ++i) wtx_absorb_byte(t, src[i]);
+    while (n > 0) {
+        const unsigned take = min(n, TX_RATE - t.hpos);
+        u64 v = 0;
+#pragma unroll
+        for (unsigned b = 0; b < 8; ++b) {
+            const unsigned i = 8 * wtx_lane() + b - t.hpos;
+            if (i < take) v |= (u64)src[i] << (8 * b);
+        }
+        t.h ^= v;
+        t.hpos += take;
+        src += take;
+        n -= take;
+        if (t.hpos == TX_RATE) {
+            t.h = keccak_f1600_warp(t.h);
+            t.hpos = 0;
+        }
+    }
 }
 
 // The first squeeze after an absorb finalises a copy of the hasher.
@@ -348,5 +366,31 @@ __device__ __forceinline__ void wtx_geometric(WarpTx& t, E3* out, int count) {
 
 // Warp-wide field sum (exact; association order free).
 __device__ __forceinline__ E3 wtx_sum(E3 v) { return e3_warp_sum(v); }
+
+// Vector RLC, constraint RLC and "the sum" (whir_prover.hpp:122-197):
+//   vrlc = geometric_challenge(V), crlc = geometric_challenge(F + O),
+//   sum  = sum_f crlc_f sum_v vrlc_v eval_(f,v) + sum_i crlc_(F+i) sum_v vrlc_v ood_(i,v)
+// over the O = nwit * ood initial OOD points, whose coordinates are also laid
+// out contiguously for the covector.  One warp.
+__device__ __forceinline__ void wtx_constraint_rlc(TxState* tx, ProofScalars* sc, int n_forms, int nwit, int ood, int nvec) {
+    const int l = wtx_lane();
+    const int n_ood = nwit * ood;
+    for (int i = l; i < n_ood; i += 32) sc->init_ood_pts[i] = sc->ood_pts[i / ood][i % ood];
+    const int count = n_forms + n_ood;
+    WarpTx t;
+    wtx_load(t, tx);
+    wtx_geometric(t, sc->vrlc, nvec);
+    wtx_geometric(t, sc->crlc, count);
+    wtx_store(t, tx);
+    E3 v = e3_zero();
+    for (int r = l; r < count; r += 32) {
+        const E3* vals = r < n_forms ? &sc->forms_eval[r * nvec] : &sc->init_ood_mat[(r - n_forms) * nvec];
+        E3 row = e3_zero();
+        for (int k = 0; k < nvec; ++k) row = e3_add(row, ef_mul(sc->vrlc[k], vals[k], t.deg == 2));
+        v = e3_add(v, ef_mul(sc->crlc[r], row, t.deg == 2));
+    }
+    v = wtx_sum(v);
+    if (l == 0) sc->sum = v;
+}
 
 }  // namespace wg
