@@ -41,3 +41,18 @@ def test_base_field_target(gpu_ctx, oracle):
     ev = np.array(gpu_ctx.mle_evaluate(coeffs, pts), dtype=np.uint64).reshape(1, 3)
     got = prove_once(n, params, coeffs, pts, ev, ctx=gpu_ctx, target_field=FIELD_GOLDILOCKS1)[:2]
     assert got == oracle.prove_forms(n, k, rho, 32, 0, [("mle", pts[0])], coeffs, ev, field1=True)
+
+
+# the single-launch form: vectors of 2^13 elements and fewer
+@pytest.mark.parametrize("n,k,rho", [
+    (17, 4, 1),  # 2^13 (the largest), 2^9, 2^5 (half a CTA's elements)
+    (14, 1, 1),  # 2^13, 2^12, ... down to one element
+    (12, 3, 3),  # few points: fewer than the warps
+])
+def test_small_vectors(gpu_ctx, oracle, n, k, rho):
+    params = ProtocolParameters.cli(folding_factor=k, log_inv_rate=rho)
+    coeffs = sample_goldilocks(650 + n + k, 1 << n)
+    pts = sample_goldilocks(660 + n, 3 * n).reshape(1, n, 3)
+    ev = np.array(gpu_ctx.mle_evaluate(coeffs, pts), dtype=np.uint64).reshape(1, 3)
+    got = prove_once(n, params, coeffs, pts, ev, ctx=gpu_ctx)[:2]
+    assert got == oracle.prove(n, k, rho, 100, 20, pts, coeffs, ev)

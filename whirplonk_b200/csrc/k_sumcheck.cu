@@ -818,57 +818,95 @@ __global__ void __launch_bounds__(256, 3) k_cov_accumulate(CovAccArgs a, const E
     }
 }
 
-// Small vectors (few pairs, tens of points): a CTA of CA_SPLIT warps over 32
-// pairs, warp w taking the points j = w, w + CA_SPLIT, ...; the partial sums
-// meet in shared memory and warp 0 adds them to the covector.  The same field
-// sums as k_cov_accumulate (exact, so the grouping is free), with the point
-// loop spread over 8x the threads: at these sizes the loop's latency, not its
-// multiply-accumulates, is the cost.
-constexpr int CA_SPLIT = 8;
-constexpr u64 CA_SPLIT_MAX_PAIRS = 2048;
-__global__ void __launch_bounds__(32 * CA_SPLIT) k_cov_accumulate_split(CovAccArgs a, const E3* tab, const u64* lo_base,
-                                                                         u32 hi_count) {
-    constexpr u32 NL = 1u << CA_LO;
-    __shared__ E3 part[CA_SPLIT][2][32];
-    const u32 per = NL + hi_count;
-    const int npts = a.n_ext + a.n_base;
-    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const u64 npair = (a.size + 1) >> 1;
-    const u64 pi = (u64)blockIdx.x * 32 + lane;
-    const u64 i = 2 * pi;
-    E3 s0 = e3_zero(), s1 = e3_zero();
-    if (pi < npair) {
-        const u32 hi = (u32)(i >> CA_LO), lo = (u32)(i & (NL - 1));  // lo even: lo + 1 < NL
-        for (int j = (int)w; j < npts; j += CA_SPLIT) {
-            const E3 h = tab[(u64)j * per + NL + hi];
-            if (j < a.n_ext) {
-                s0 = e3_add(s0, e3_mul(h, tab[(u64)j * per + lo]));
-                s1 = e3_add(s1, e3_mul(h, tab[(u64)j * per + lo + 1]));
-            } else {
-                const u64* lb = lo_base + (u64)(j - a.n_ext) * NL + lo;
-                s0 = e3_add(s0, e3_mul_base(h, lb[0]));
-                s1 = e3_add(s1, e3_mul_base(h, lb[1]));
+// Vectors of up to 2^13 elements, in one launch without tables: a CTA of CS_WARPS + 1
+// warps owns 64 elements, 64 c .. 64 c + 63, lane l the elements l and l + 32 of
+// them.  A warp takes every CS_WARPS-th base point, two at a time, and forms its
+// powers itself: z^l by the bits of its lane, z^32 as the last of those squarings,
+// z^(64 c) by the bits of c.  The last warp takes the Ext3 points.  The warps' sums
+// meet in shared memory.
+//
+// Bound by its ~14 products a point and lane (an SM at 4 warps a scheduler), with many
+// points on few CTAs.  The tables took a launch of their own (powers of up to 12 bits,
+// serial) and the sums two L2 loads a point and element: B200, all updates of a proof,
+// before and now: n = 12 53 -> 48 us, n = 16 63 -> 55, n = 20 88 -> 74.
+constexpr int CS_WARPS = 16;
+constexpr u64 CS_MAX = 1ull << 13;
+__global__ void __launch_bounds__(32 * (CS_WARPS + 1), 1) k_cov_small(const __grid_constant__ CovAccArgs a) {
+    __shared__ u64 sums[CS_WARPS + 1][6][32];
+    const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x;
+    E3 s0 = e3_zero(), s1 = e3_zero();  // elements lane, lane + 32
+    if (w < (u32)CS_WARPS) {
+        E3AccL b0{}, b1{};
+        for (int j = (int)w; j < a.n_base; j += 2 * CS_WARPS) {
+            u64 z[2], r[2], t[2];
+            E3 rl[2];
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int q = a.n_ext + j + p * CS_WARPS;
+                const bool on = j + p * CS_WARPS < a.n_base;
+                z[p] = on ? a.sc->stir_pts[q].c0 : 0;
+                rl[p] = on ? a.sc->stir_rlc[q] : e3_zero();
+                r[p] = t[p] = 1;
+            }
+#pragma unroll 1
+            for (u32 b = 0; b < 5; ++b)
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    const u64 m = gl_mul(r[p], z[p]);
+                    if ((lane >> b) & 1) r[p] = m;
+                    z[p] = gl_mul(z[p], z[p]);
+                }
+            const u64 z32[2] = {z[0], z[1]};
+#pragma unroll 1
+            for (u32 e = 2 * c; e; e >>= 1)
+#pragma unroll
+                for (int p = 0; p < 2; ++p) {
+                    if (e & 1) t[p] = gl_mul(t[p], z[p]);
+                    z[p] = gl_mul(z[p], z[p]);
+                }
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const u64 x = gl_mul(r[p], t[p]), y = gl_mul(x, z32[p]);
+                accl_mac_base(b0, x, rl[p]);
+                accl_mac_base(b1, y, rl[p]);
             }
         }
-    }
-    part[w][0][lane] = s0;
-    part[w][1][lane] = s1;
-    __syncthreads();
-    if (w != 0 || pi >= npair) return;
+        s0 = accl_reduce(b0);
+        s1 = accl_reduce(b1);
+    } else {
+        for (int j = 0; j < a.n_ext; ++j) {
+            E3 z = a.sc->stir_pts[j], r = e3_one(), t = a.sc->stir_rlc[j];
 #pragma unroll 1
-    for (int k = 1; k < CA_SPLIT; ++k) {
-        s0 = e3_add(s0, part[k][0][lane]);
-        s1 = e3_add(s1, part[k][1][lane]);
+            for (u32 b = 0; b < 5; ++b) {
+                const E3 m = ef_mul(r, z, a.ext2);
+                if ((lane >> b) & 1) r = m;
+                z = ef_mul(z, z, a.ext2);
+            }
+            const E3 z32 = z;
+#pragma unroll 1
+            for (u32 e = 2 * c; e; e >>= 1) {
+                if (e & 1) t = ef_mul(t, z, a.ext2);
+                z = ef_mul(z, z, a.ext2);
+            }
+            r = ef_mul(r, t, a.ext2);
+            s0 = e3_add(s0, r);
+            s1 = e3_add(s1, ef_mul(r, z32, a.ext2));
+        }
     }
-    s0 = ef_fix(s0, a.ext2);
-    s1 = ef_fix(s1, a.ext2);
-    a.cov[0][i] = gl_add(a.cov[0][i], s0.c0);
-    a.cov[1][i] = gl_add(a.cov[1][i], s0.c1);
-    a.cov[2][i] = gl_add(a.cov[2][i], s0.c2);
-    if (i + 1 < a.size) {
-        a.cov[0][i + 1] = gl_add(a.cov[0][i + 1], s1.c0);
-        a.cov[1][i + 1] = gl_add(a.cov[1][i + 1], s1.c1);
-        a.cov[2][i + 1] = gl_add(a.cov[2][i + 1], s1.c2);
+    sums[w][0][lane] = s0.c0;
+    sums[w][1][lane] = s0.c1;
+    sums[w][2][lane] = s0.c2;
+    sums[w][3][lane] = s1.c0;
+    sums[w][4][lane] = s1.c1;
+    sums[w][5][lane] = s1.c2;
+    __syncthreads();
+    if (w < 6) {  // component w mod 3 of 32 elements
+        const u64 i = 64ull * c + (w < 3 ? 0 : 32) + lane;
+        u64 v = sums[0][w][lane];
+#pragma unroll
+        for (int k = 1; k <= CS_WARPS; ++k) v = gl_add(v, sums[k][w][lane]);
+        u64* cov = a.cov[w < 3 ? w : w - 3];
+        if (i < a.size) cov[i] = gl_add(cov[i], v);
     }
 }
 
@@ -884,20 +922,20 @@ int launch_cov_accumulate(const CovAccArgs& a, cudaStream_t st) {
     if (npts == 0 || a.size == 0) return 0;
     const int rc = launch_cov_gemm(a, st);
     if (rc != 1) return rc;
+    for (int c = 0; c < 3; ++c)
+        if (reinterpret_cast<uintptr_t>(a.cov[c]) & 15) return -1;  // 16-byte pairs
+    if (a.size <= CS_MAX) {
+        k_cov_small<<<(unsigned)((a.size + 63) / 64), 32 * (CS_WARPS + 1), 0, st>>>(a);
+        count_launches(1);
+        return 0;
+    }
     const u32 hc = ca_hi_count(a.size);
     E3* tab = reinterpret_cast<E3*>(a.scratch);
     const size_t tab_bytes = ((size_t)(1u << CA_LO) + hc) * (size_t)npts * sizeof(E3);
     u64* lo_base = reinterpret_cast<u64*>(reinterpret_cast<char*>(a.scratch) + (tab_bytes + 255) / 256 * 256);
     k_cov_acc_tables<<<2 * device_sms(), 256, 0, st>>>(a.sc, a.n_ext, npts, hc, tab, lo_base, a.ext2 != 0);
     count_launches(1);
-    for (int c = 0; c < 3; ++c)
-        if (reinterpret_cast<uintptr_t>(a.cov[c]) & 15) return -1;  // 16-byte pairs
     const u64 npair = (a.size + 1) / 2;
-    if (npair <= CA_SPLIT_MAX_PAIRS) {
-        k_cov_accumulate_split<<<(unsigned)((npair + 31) / 32), 32 * CA_SPLIT, 0, st>>>(a, tab, lo_base, hc);
-        count_launches(1);
-        return 0;
-    }
     u64 want = (npair + 255) / 256;
     const u64 cap = (u64)device_sms() * 16;
     k_cov_accumulate<<<(unsigned)(want > cap ? cap : want), 256, 0, st>>>(a, tab, lo_base, hc);
