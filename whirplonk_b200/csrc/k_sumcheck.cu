@@ -820,56 +820,61 @@ __global__ void __launch_bounds__(256, 3) k_cov_accumulate(CovAccArgs a, const E
 
 // Vectors of up to 2^13 elements, in one launch without tables: a CTA of CS_WARPS + 1
 // warps owns 64 elements, 64 c .. 64 c + 63, lane l the elements l and l + 32 of
-// them.  A warp takes every CS_WARPS-th base point, two at a time, and forms its
-// powers itself: z^l by the bits of its lane, z^32 as the last of those squarings,
-// z^(64 c) by the bits of c.  The last warp takes the Ext3 points.  The warps' sums
-// meet in shared memory.
+// them.  A warp takes every CS_WARPS-th base point, CS_BATCH of them at a time: first
+// a lane a point forms z, z^2, .. z^16 and the coefficients rlc z^(64 c) and
+// rlc z^(64 c + 32), then every lane its z^l of each point (four products) and the two
+// sums.  The last warp takes the Ext3 points.  The warps' sums meet in shared memory.
 //
-// Bound by its ~14 products a point and lane (an SM at 4 warps a scheduler), with many
-// points on few CTAs.  The tables took a launch of their own (powers of up to 12 bits,
-// serial) and the sums two L2 loads a point and element: B200, all updates of a proof,
-// before and now: n = 12 53 -> 48 us, n = 16 63 -> 55, n = 20 88 -> 74.
-constexpr int CS_WARPS = 16;
+// Bound by the ~150 instructions a point and warp, with many points on few CTAs.  The
+// tables took a launch of their own (powers of up to 12 bits, serial) and the sums two
+// L2 loads a point and element: B200, all updates of a proof, before and now:
+// n = 12 53 -> 32 us, n = 16 63 -> 46, n = 20 88 -> 70.
+// (Each lane forming z^l and z^(64 c) from z alone: ~500 instructions, 48 us at n = 12.)
+constexpr int CS_WARPS = 16, CS_BATCH = 16;
 constexpr u64 CS_MAX = 1ull << 13;
 __global__ void __launch_bounds__(32 * (CS_WARPS + 1), 1) k_cov_small(const __grid_constant__ CovAccArgs a) {
-    __shared__ u64 sums[CS_WARPS + 1][6][32];
+    __shared__ u64 buf[(CS_WARPS + 1) * 6 * 32];
+    u64(*sums)[6][32] = reinterpret_cast<u64(*)[6][32]>(buf);
     const u32 lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x;
     E3 s0 = e3_zero(), s1 = e3_zero();  // elements lane, lane + 32
     if (w < (u32)CS_WARPS) {
+        static_assert(CS_WARPS * CS_BATCH * 11 <= (CS_WARPS + 1) * 6 * 32, "the points' words fit the sums' place");
+        u64(*pt)[11] = reinterpret_cast<u64(*)[11]>(buf + w * CS_BATCH * 11);
         E3AccL b0{}, b1{};
-        for (int j = (int)w; j < a.n_base; j += 2 * CS_WARPS) {
-            u64 z[2], r[2], t[2];
-            E3 rl[2];
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const int q = a.n_ext + j + p * CS_WARPS;
-                const bool on = j + p * CS_WARPS < a.n_base;
-                z[p] = on ? a.sc->stir_pts[q].c0 : 0;
-                rl[p] = on ? a.sc->stir_rlc[q] : e3_zero();
-                r[p] = t[p] = 1;
-            }
+        for (int j0 = (int)w; j0 < a.n_base; j0 += CS_BATCH * CS_WARPS) {
+            const int left = (a.n_base - j0 + CS_WARPS - 1) / CS_WARPS, cnt = left < CS_BATCH ? left : CS_BATCH;
+            if ((int)lane < cnt) {
+                const int q = a.n_ext + j0 + (int)lane * CS_WARPS;
+                u64 z = a.sc->stir_pts[q].c0, t = 1;
+                const E3 rl = a.sc->stir_rlc[q];
 #pragma unroll 1
-            for (u32 b = 0; b < 5; ++b)
-#pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    const u64 m = gl_mul(r[p], z[p]);
-                    if ((lane >> b) & 1) r[p] = m;
-                    z[p] = gl_mul(z[p], z[p]);
+                for (u32 b = 0; b < 5; ++b) {
+                    pt[lane][b] = z;
+                    z = gl_mul(z, z);
                 }
-            const u64 z32[2] = {z[0], z[1]};
+                const u64 z32 = z;
 #pragma unroll 1
-            for (u32 e = 2 * c; e; e >>= 1)
-#pragma unroll
-                for (int p = 0; p < 2; ++p) {
-                    if (e & 1) t[p] = gl_mul(t[p], z[p]);
-                    z[p] = gl_mul(z[p], z[p]);
+                for (u32 e = 2 * c; e; e >>= 1) {
+                    if (e & 1) t = gl_mul(t, z);
+                    z = gl_mul(z, z);
                 }
-#pragma unroll
-            for (int p = 0; p < 2; ++p) {
-                const u64 x = gl_mul(r[p], t[p]), y = gl_mul(x, z32[p]);
-                accl_mac_base(b0, x, rl[p]);
-                accl_mac_base(b1, y, rl[p]);
+                const E3 r0 = e3_mul_base(rl, t), r1 = e3_mul_base(r0, z32);
+                pt[lane][5] = r0.c0;
+                pt[lane][6] = r0.c1;
+                pt[lane][7] = r0.c2;
+                pt[lane][8] = r1.c0;
+                pt[lane][9] = r1.c1;
+                pt[lane][10] = r1.c2;
             }
+            __syncwarp();
+#pragma unroll 2
+            for (int p = 0; p < cnt; ++p) {
+                auto pick = [&](u32 b) { return ((lane >> b) & 1) ? pt[p][b] : 1ull; };
+                const u64 x = gl_mul(gl_mul(gl_mul(pick(0), pick(1)), gl_mul(pick(2), pick(3))), pick(4));
+                accl_mac_base(b0, x, E3{pt[p][5], pt[p][6], pt[p][7]});
+                accl_mac_base(b1, x, E3{pt[p][8], pt[p][9], pt[p][10]});
+            }
+            __syncwarp();
         }
         s0 = accl_reduce(b0);
         s1 = accl_reduce(b1);
@@ -893,6 +898,7 @@ __global__ void __launch_bounds__(32 * (CS_WARPS + 1), 1) k_cov_small(const __gr
             s1 = e3_add(s1, ef_mul(r, z32, a.ext2));
         }
     }
+    __syncthreads();  // the points' words have been read
     sums[w][0][lane] = s0.c0;
     sums[w][1][lane] = s0.c1;
     sums[w][2][lane] = s0.c2;
