@@ -292,7 +292,6 @@ __device__ __forceinline__ E3 wtx_challenges(WarpTx& t, u32 ncomp) {
     return E3{c0, ncomp > 1 ? c1 : 0, ncomp > 2 ? c2 : 0};
 }
 __device__ __forceinline__ u64 wtx_challenge_base(WarpTx& t) { return wtx_challenges(t, 1).c0; }
-__device__ __forceinline__ E3 wtx_challenge_e3(WarpTx& t) { return wtx_challenges(t, 3); }
 
 // Elements of the protocol's target field.  With the base field as target
 // (Identity<Goldilocks>) its elements are carried as Ext3 values (x, 0, 0) --
