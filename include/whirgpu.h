@@ -413,6 +413,10 @@ whirgpu_status whirgpu_mle_evaluate_noalloc(const uint64_t* d_coeffs, uint64_t n
  * (op 0: a+b, 1: a-b, 2: a*b in Goldilocks; 3: a*b in Ext3, three words per
  * element) and copies the results back.  Operands must be canonical. */
 whirgpu_status whirgpu_debug_field_ops(const uint64_t* a, const uint64_t* b, uint64_t* out, uint64_t n, int op);
+/* Diagnostics: fills the device blocks that the context keeps for its next
+ * zero-knowledge witnesses with `byte` (blocks: how many), so a test can show
+ * that a proof reads nothing of them that it has not written. */
+whirgpu_status whirgpu_debug_fill_zk_pool(whirgpu_ctx* ctx, int byte, size_t* blocks);
 /* Seeded uniform Goldilocks words: ChaCha20 block function (RFC 8439),
  * key = seed as 8 LE bytes then 24 zero bytes, nonce 0, counter from 0;
  * each 64-bit LE keystream word below p is taken, others are skipped. */

@@ -26,7 +26,7 @@ EXPORTED = [
     "whirgpu_workspace_bytes",
     "whirgpu_cli_domain_separator", "whirgpu_transcript_create", "whirgpu_transcript_destroy", "whirgpu_proof_get",
     "whirgpu_commit", "whirgpu_commit_witnesses", "whirgpu_config_from_params", "whirgpu_commit_config", "whirgpu_witness_destroy", "whirgpu_prove", "whirgpu_prove_forms", "whirgpu_mle_evaluate", "whirgpu_mle_evaluate_noalloc",
-    "whirgpu_debug_field_ops", "whirgpu_sample_goldilocks", "whirgpu_chacha20_block", "whirgpu_host_alloc", "whirgpu_host_free",
+    "whirgpu_debug_field_ops", "whirgpu_debug_fill_zk_pool", "whirgpu_sample_goldilocks", "whirgpu_chacha20_block", "whirgpu_host_alloc", "whirgpu_host_free",
     "whirgpu_set_timing", "whirgpu_kernel_stats", "whirgpu_launch_count", "whirgpu_last_io_bytes",
     "whirgpu_workspace_stats",
     "whirgpu_measure_int_peaks",
@@ -196,6 +196,8 @@ def load() -> ctypes.CDLL:
     L.whirgpu_mle_evaluate.argtypes = [p, p, u64, i32, p, p]
     L.whirgpu_mle_evaluate_noalloc.argtypes = [p, u64, p, p, p]
     L.whirgpu_debug_field_ops.argtypes = [p, p, p, u64, i32]
+    L.whirgpu_debug_fill_zk_pool.argtypes = [p, i32, ctypes.POINTER(sz)]
+    L.whirgpu_debug_fill_zk_pool.restype = i32
     L.whirgpu_sample_goldilocks.argtypes = [u64, p, sz]
     L.whirgpu_sample_goldilocks.restype = None
     L.whirgpu_chacha20_block.argtypes = [p, ctypes.c_uint32, p, p]

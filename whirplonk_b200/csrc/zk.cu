@@ -620,12 +620,17 @@ whirgpu_status whirgpu_zk_commit(whirgpu_ctx* c, const whirgpu_zk_config* cfg, c
         w->dev = nullptr;
         return zk_fail(c, s, m);
     };
-    // Counters and tickets of both workspaces start at zero (they reset
-    // themselves after use, as in the workspace cache).
-    cudaError_t e = cudaMemsetAsync(dev + w->off_b + w->pb.off_sc_scratch, 0, w->pb.off_tx - w->pb.off_sc_scratch,
-                                    c->stream);
-    if (e == cudaSuccess)
-        e = cudaMemsetAsync(dev + w->off_g + w->pg.off_sc_scratch, 0, w->pg.off_tx - w->pg.off_sc_scratch, c->stream);
+    // Counters and tickets of both workspaces start at zero (they reset themselves
+    // after use, as in the workspace cache): those in the scratch regions and the
+    // ProofScalars' (the transcript's start clears them in one workspace only, and
+    // the two proofs share one transcript).
+    auto clear_tickets = [&](const ProofPlan& p, char* ws) -> cudaError_t {
+        const cudaError_t e1 = cudaMemsetAsync(ws + p.off_sc_scratch, 0, p.off_tx - p.off_sc_scratch, c->stream);
+        if (e1 != cudaSuccess) return e1;
+        return cudaMemsetAsync(plan_scalars(p, ws)->counters, 0, sizeof(ProofScalars::counters), c->stream);
+    };
+    cudaError_t e = clear_tickets(w->pb, dev + w->off_b);
+    if (e == cudaSuccess) e = clear_tickets(w->pg, dev + w->off_g);
     TxState* txs = reinterpret_cast<TxState*>(dev + w->off_tx);
     w->pb.tx_ext = txs;
     w->pg.tx_ext = txs;
@@ -882,6 +887,19 @@ whirgpu_status whirgpu_zk_prove(whirgpu_ctx* c, whirgpu_zk_witness* w, const whi
     ZK_CUDA(c, cudaStreamSynchronize(st), "read-back");
     c->io_d2h += sizeof(TxState) + htx.narg_len + htx.hints_len;
     tx->complete = true;
+    return WHIRGPU_OK;
+}
+
+whirgpu_status whirgpu_debug_fill_zk_pool(whirgpu_ctx* c, int byte, size_t* blocks) {
+    if (!c || !blocks) return WHIRGPU_E_INVALID;
+    *blocks = 0;
+    std::lock_guard<std::recursive_mutex> lk(c->cache_mu);
+    for (auto& kv : c->zk_pool)
+        for (char* p : kv.second) {
+            ZK_CUDA(c, cudaMemsetAsync(p, byte, kv.first, c->stream), "fill pool");
+            ++*blocks;
+        }
+    ZK_CUDA(c, cudaStreamSynchronize(c->stream), "fill pool");
     return WHIRGPU_OK;
 }
 
