@@ -332,14 +332,21 @@ void whirgpu_server_destroy(whirgpu_server* s);
  * i < N = 2^log_expansion m, w_N = 7^((p-1)/N).  Device pointers only: the
  * vectors back to back; d_tmp and d_planes hold count * 2^log_depth * N words
  * each; plane (vector k, block b) = d_planes + (k 2^log_depth + b) N.
- * Enqueued on the context stream (whirgpu_stream); returns without waiting. */
+ * Enqueued on the context stream (whirgpu_stream); returns without waiting.  The
+ * waits inside its kernels are bounded; should one run out, the planes are
+ * incomplete and the next whirgpu_rs_encode (which then enqueues nothing) or
+ * whirgpu_rs_encode_status of the context returns WHIRGPU_E_DEVICE, once. */
 whirgpu_status whirgpu_rs_encode(whirgpu_ctx* ctx, const uint64_t* d_vectors, size_t count, uint32_t log_len,
                                  uint32_t log_expansion, uint32_t log_depth, uint64_t* d_tmp, uint64_t* d_planes);
+/* Waits for the context stream: WHIRGPU_OK when every encode so far is complete
+ * or has been reported, else WHIRGPU_E_DEVICE (see above). */
+whirgpu_status whirgpu_rs_encode_status(whirgpu_ctx* ctx);
 /* RS-encode and Merkle-commit `count` vectors (host or device memory, see
  * WHIRGPU_INPUT_*): per vector the root of irs_commit::commit's matrix
  * commitment (rows of 2^log_depth elements, leaf = BLAKE3 of the row's LE bytes,
  * matrix_commit.hpp:169-195; tree merkle_tree.hpp:104-147), written to
- * roots[32 k ..].  Synchronous.  Replaces the commitment half of
+ * roots[32 k ..].  Synchronous; WHIRGPU_E_DEVICE when a bounded wait of this
+ * call's kernels ran out.  Replaces the commitment half of
  * Config::commit (irs_commit.hpp:433-470) for many vectors at once, without the
  * transcript. */
 whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* ctx, const uint64_t* vectors, int location, size_t count,
@@ -417,6 +424,9 @@ whirgpu_status whirgpu_debug_field_ops(const uint64_t* a, const uint64_t* b, uin
  * zero-knowledge witnesses with `byte` (blocks: how many), so a test can show
  * that a proof reads nothing of them that it has not written. */
 whirgpu_status whirgpu_debug_fill_zk_pool(whirgpu_ctx* ctx, int byte, size_t* blocks);
+/* Diagnostics: a bounded wait (about two seconds) that nothing ends, recorded as
+ * a wait of an encode's kernels or (commit != 0) of a commitment's. */
+whirgpu_status whirgpu_debug_expire_wait(whirgpu_ctx* ctx, int commit);
 /* Seeded uniform Goldilocks words: ChaCha20 block function (RFC 8439),
  * key = seed as 8 LE bytes then 24 zero bytes, nonce 0, counter from 0;
  * each 64-bit LE keystream word below p is taken, others are skipped. */

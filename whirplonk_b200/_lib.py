@@ -26,14 +26,14 @@ EXPORTED = [
     "whirgpu_workspace_bytes",
     "whirgpu_cli_domain_separator", "whirgpu_transcript_create", "whirgpu_transcript_destroy", "whirgpu_proof_get",
     "whirgpu_commit", "whirgpu_commit_witnesses", "whirgpu_config_from_params", "whirgpu_commit_config", "whirgpu_witness_destroy", "whirgpu_prove", "whirgpu_prove_forms", "whirgpu_mle_evaluate", "whirgpu_mle_evaluate_noalloc",
-    "whirgpu_debug_field_ops", "whirgpu_debug_fill_zk_pool", "whirgpu_sample_goldilocks", "whirgpu_chacha20_block", "whirgpu_host_alloc", "whirgpu_host_free",
+    "whirgpu_debug_field_ops", "whirgpu_debug_fill_zk_pool", "whirgpu_debug_expire_wait", "whirgpu_sample_goldilocks", "whirgpu_chacha20_block", "whirgpu_host_alloc", "whirgpu_host_free",
     "whirgpu_set_timing", "whirgpu_kernel_stats", "whirgpu_launch_count", "whirgpu_last_io_bytes",
     "whirgpu_workspace_stats",
     "whirgpu_measure_int_peaks",
     "whirgpu_batch_create", "whirgpu_batch_run", "whirgpu_batch_proof", "whirgpu_batch_destroy",
     "whirgpu_server_create", "whirgpu_server_submit", "whirgpu_server_poll", "whirgpu_server_release",
     "whirgpu_server_stats", "whirgpu_server_destroy",
-    "whirgpu_rs_encode", "whirgpu_rs_commit_batch",
+    "whirgpu_rs_encode", "whirgpu_rs_encode_status", "whirgpu_rs_commit_batch",
     "whirgpu_ntt_autotune", "whirgpu_ntt_set_plan", "whirgpu_ntt_get_plan", "whirgpu_ntt_clear_plans",
     "whirgpu_ntt_list_plans", "whirgpu_ntt_load_plans", "whirgpu_ntt_save_plans", "whirgpu_ntt_load_default_plans",
     "whirgpu_zk_config_from_params", "whirgpu_zk_commit", "whirgpu_zk_prove", "whirgpu_zk_witness_destroy",
@@ -198,6 +198,8 @@ def load() -> ctypes.CDLL:
     L.whirgpu_debug_field_ops.argtypes = [p, p, p, u64, i32]
     L.whirgpu_debug_fill_zk_pool.argtypes = [p, i32, ctypes.POINTER(sz)]
     L.whirgpu_debug_fill_zk_pool.restype = i32
+    L.whirgpu_debug_expire_wait.argtypes = [p, i32]
+    L.whirgpu_debug_expire_wait.restype = i32
     L.whirgpu_sample_goldilocks.argtypes = [u64, p, sz]
     L.whirgpu_sample_goldilocks.restype = None
     L.whirgpu_chacha20_block.argtypes = [p, ctypes.c_uint32, p, p]
@@ -234,6 +236,8 @@ def load() -> ctypes.CDLL:
     L.whirgpu_server_destroy.restype = None
     u32 = ctypes.c_uint32
     L.whirgpu_rs_encode.argtypes = [p, p, sz, u32, u32, u32, p, p]
+    L.whirgpu_rs_encode_status.argtypes = [p]
+    L.whirgpu_rs_encode_status.restype = i32
     L.whirgpu_rs_commit_batch.argtypes = [p, p, i32, sz, u32, u32, u32, p]
     L.whirgpu_ntt_autotune.argtypes = [p, u32, u32, u32, u32, ctypes.POINTER(NttPlan),
                                        ctypes.POINTER(ctypes.c_double), ctypes.POINTER(u32)]

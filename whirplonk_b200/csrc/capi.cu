@@ -323,8 +323,9 @@ whirgpu_status whirgpu_ctx_create(int device, uint64_t hbm_budget, whirgpu_ctx**
     WG_CUDA(nullptr, cudaMemcpy(c->tw.tw_hi, hi.data(), hi.size() * 8, cudaMemcpyHostToDevice), "upload");
     WG_CUDA(nullptr, cudaMemcpy(c->tw.tw_lo, lo.data(), lo.size() * 8, cudaMemcpyHostToDevice), "upload");
     c->tw.lde = &c->lde_tables;
-    WG_CUDA(nullptr, cudaHostAlloc(&c->lde_err, sizeof(uint32_t), cudaHostAllocMapped), "cudaHostAlloc");
-    *c->lde_err = 0;
+    WG_CUDA(nullptr, cudaHostAlloc(&c->kernel_err, whirgpu_ctx::ERR_WORDS * sizeof(uint32_t), cudaHostAllocMapped),
+            "cudaHostAlloc");
+    std::memset(c->kernel_err, 0, whirgpu_ctx::ERR_WORDS * sizeof(uint32_t));
     *out = c.release();
     return WHIRGPU_OK;
 }
@@ -348,7 +349,7 @@ void whirgpu_ctx_destroy(whirgpu_ctx* c) {
     cudaFree(c->tw.tw_hi);
     cudaFree(c->tw.tw_lo);
     lde_tables_free(c->lde_tables);
-    if (c->lde_err) cudaFreeHost(c->lde_err);
+    if (c->kernel_err) cudaFreeHost(c->kernel_err);
     if (c->pinned) cudaFreeHost(c->pinned);
     if (c->mle_scratch) cudaFree(c->mle_scratch);
     if (c->kscratch) cudaFree(c->kscratch);

@@ -99,7 +99,12 @@ struct whirgpu_ctx {
     uint64_t ws_allocations = 0, ws_evictions = 0;  // workspaces allocated / freed to make room
     wg::DeviceTables tw;
     wg::LdeTables lde_tables;  // inter-pass twiddle factors of the LDE splits in use (tw.lde)
-    uint32_t* lde_err = nullptr;  // pinned, mapped: error bits of the kernel-level encoder calls
+    // Error bits of the kernel-level calls (pinned, mapped): a word for the encodes
+    // that have not reported yet, one for the commitment under way.
+    enum { ERR_ENCODE = 0, ERR_COMMIT = 1, ERR_WORDS = 2 };
+    uint32_t* kernel_err = nullptr;
+    // The bits of one word, which start over at zero: each failure is reported once.
+    uint32_t take_kernel_err(int which) { return __atomic_exchange_n(kernel_err + which, 0u, __ATOMIC_ACQ_REL); }
     std::string err;
     // Workspaces by plan shape: the schedule, hash engine, vector layout, field
     // degree and domain-separator length, serialised (plan_key).

@@ -3,8 +3,11 @@
 #include <cuda_runtime.h>
 
 #include "../../include/whirgpu.h"
+#include "ctx.h"
 #include "gl.cuh"
+#include "i8mma.cuh"
 #include "launch.h"
+#include "transcript.cuh"
 
 namespace wg {
 
@@ -24,7 +27,24 @@ __global__ void k_field_ops(const u64* a, const u64* b, u64* out, u64 n, int op)
     }
 }
 
+// Waits for a barrier that nothing arrives at, with the kernels' own bounded wait.
+__global__ void k_expire_wait(u32* err) {
+    __shared__ __align__(8) u64 bar;
+    mbar_init(smem_u32(&bar), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (!mbar_wait(smem_u32(&bar), 0)) atomicOr_system(err, TX_ERR_TIMEOUT);
+}
+
 }  // namespace wg
+
+extern "C" whirgpu_status whirgpu_debug_expire_wait(whirgpu_ctx* c, int commit) {
+    using namespace wg;
+    if (!c) return WHIRGPU_E_INVALID;
+    k_expire_wait<<<1, 1, 0, c->stream>>>(c->kernel_err + (commit ? whirgpu_ctx::ERR_COMMIT : whirgpu_ctx::ERR_ENCODE));
+    count_launches(1);
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    return e == cudaSuccess ? WHIRGPU_OK : cuda_fail(c, e, "expiring wait");
+}
 
 extern "C" whirgpu_status whirgpu_debug_field_ops(const uint64_t* a, const uint64_t* b, uint64_t* out, uint64_t n,
                                                   int op) {

@@ -85,7 +85,7 @@ whirgpu_status kernel_scratch(whirgpu_ctx* c, size_t bytes, char** out) {
     return WHIRGPU_OK;
 }
 
-LdeArgs lde_args(whirgpu_ctx* c, const u64* src, u64 m, u32 planes, u32 logN, u64* tmp, u64* out) {
+LdeArgs lde_args(whirgpu_ctx* c, const u64* src, u64 m, u32 planes, u32 logN, u64* tmp, u64* out, u32* err) {
     LdeArgs L{};
     L.src[0] = L.src[1] = L.src[2] = src;
     L.m = m;
@@ -98,7 +98,7 @@ LdeArgs lde_args(whirgpu_ctx* c, const u64* src, u64 m, u32 planes, u32 logN, u6
     L.tw_hi = c->tw.tw_hi;
     L.tw_lo = c->tw.tw_lo;
     L.tables = &c->lde_tables;
-    L.err = c->lde_err;
+    L.err = err;
     return L;
 }
 
@@ -120,6 +120,8 @@ void prepare_plan_tables(whirgpu_ctx* c, const LdePlan& pl) {
     lde_tables_prepare_plan(c->lde_tables, pl, c->tw.tw_hi, c->tw.tw_lo, c->stream, room);
 }
 
+constexpr const char* ENCODE_LATE = "a bounded wait of an earlier encode's kernels ran out: its planes are incomplete";
+
 bool shape_ok(uint32_t log_len, uint32_t log_expansion, uint32_t log_depth) {
     return log_depth <= 6 && log_len >= log_depth && log_len <= 30 && log_expansion <= 16 &&
            log_len - log_depth + log_expansion <= TW_LOG;
@@ -139,11 +141,21 @@ whirgpu_status whirgpu_rs_encode(whirgpu_ctx* c, const uint64_t* d_vectors, size
     const u64 planes = (u64)count << log_depth;
     if (planes > 65535) return fail(c, WHIRGPU_E_INVALID, "too many planes");
     const u32 logN = log_len - log_depth + log_expansion;
+    // An encode returns before its kernels run: what it could not report, this call does.
+    if (c->take_kernel_err(whirgpu_ctx::ERR_ENCODE)) return fail(c, WHIRGPU_E_DEVICE, ENCODE_LATE);
     prepare_shape_tables(c, logN, log_expansion, (u32)planes, d_vectors, d_tmp);
-    const LdeArgs L = lde_args(c, d_vectors, 1ull << (log_len - log_depth), (u32)planes, logN, d_tmp, d_planes);
+    const LdeArgs L = lde_args(c, d_vectors, 1ull << (log_len - log_depth), (u32)planes, logN, d_tmp, d_planes,
+                               c->kernel_err + whirgpu_ctx::ERR_ENCODE);
     if (launch_lde(L, c->stream) != 0) return fail(c, WHIRGPU_E_INVALID, "LDE launch");
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? WHIRGPU_OK : cuda_fail(c, e, "LDE");
+}
+
+whirgpu_status whirgpu_rs_encode_status(whirgpu_ctx* c) {
+    if (!c) return WHIRGPU_E_INVALID;
+    const cudaError_t e = cudaStreamSynchronize(c->stream);
+    if (e != cudaSuccess) return cuda_fail(c, e, "encode");
+    return c->take_kernel_err(whirgpu_ctx::ERR_ENCODE) ? fail(c, WHIRGPU_E_DEVICE, ENCODE_LATE) : WHIRGPU_OK;
 }
 
 whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* c, const uint64_t* vectors, int location, size_t count,
@@ -172,10 +184,11 @@ whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* c, const uint64_t* vectors, 
         if (e != cudaSuccess) return cuda_fail(c, e, "input copy");
         src = in;
     }
-    const LdeArgs L = lde_args(c, src, 1ull << (log_len - log_depth), (u32)planes, logN, tmp, out);
+    u32* const err = c->kernel_err + whirgpu_ctx::ERR_COMMIT;
+    const LdeArgs L = lde_args(c, src, 1ull << (log_len - log_depth), (u32)planes, logN, tmp, out, err);
     if (launch_lde(L, c->stream) != 0) return fail(c, WHIRGPU_E_INVALID, "LDE launch");
     const u32 depth = 1u << log_depth;
-    if (launch_leaves_batch(out, N, depth, 1, nodes, (u32)count, (u64)depth * N, node_words, 0, c->stream, 0, c->lde_err) != 0)
+    if (launch_leaves_batch(out, N, depth, 1, nodes, (u32)count, (u64)depth * N, node_words, 0, c->stream, 0, err) != 0)
         return fail(c, WHIRGPU_E_INVALID, "leaf launch");
     if (launch_merkle_batch(nodes, logN, (u32)count, node_words, c->stream) != 0)
         return fail(c, WHIRGPU_E_INVALID, "merkle launch");
@@ -188,7 +201,8 @@ whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* c, const uint64_t* vectors, 
     if (ec != cudaSuccess) return cuda_fail(c, ec, "root copy");
     const cudaError_t e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "rs_commit");
-    if (*(volatile uint32_t*)c->lde_err) return fail(c, WHIRGPU_E_DEVICE, "encoder wait ran out");
+    if (c->take_kernel_err(whirgpu_ctx::ERR_COMMIT))
+        return fail(c, WHIRGPU_E_DEVICE, "a bounded wait of this commitment's kernels ran out");
     return WHIRGPU_OK;
 }
 
@@ -207,7 +221,7 @@ whirgpu_status whirgpu_ntt_autotune(whirgpu_ctx* c, uint32_t log_n, uint32_t log
     u64* src = out + planes * N;
     unsigned long long* dig = reinterpret_cast<unsigned long long*>(src + planes * m);
     k_fill_canonical<<<4 * device_sms(), 256, 0, c->stream>>>(src, planes * m, 0x5EED0000ull + log_n);
-    const LdeArgs L = lde_args(c, src, m, planes, log_n, tmp, out);
+    const LdeArgs L = lde_args(c, src, m, planes, log_n, tmp, out, nullptr);  // butterfly passes wait for nothing
 
     auto digest = [&](unsigned long long* h) -> bool {
         cudaMemsetAsync(dig, 0, 8, c->stream);

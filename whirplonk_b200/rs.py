@@ -46,6 +46,13 @@ def rs_commit_batch(ctx: Context, vectors, log_expansion: int, log_depth: int = 
 def rs_encode(ctx: Context, d_vectors: int, count: int, log_len: int, log_expansion: int, log_depth: int,
               d_tmp: int, d_planes: int) -> None:
     """Enqueues the encoder on the context stream (device pointers; see
-    whirgpu_rs_encode for the plane layout)."""
+    whirgpu_rs_encode for the plane layout).  Raises with E_DEVICE, and enqueues
+    nothing, when an earlier encode turned out incomplete."""
     _lib.check(_lib.load().whirgpu_rs_encode(ctx.handle, d_vectors, count, log_len, log_expansion, log_depth, d_tmp,
                                               d_planes), ctx.handle)
+
+
+def rs_encode_status(ctx: Context) -> None:
+    """Waits for the context stream; raises with E_DEVICE when an encode enqueued
+    since the last report is incomplete (a bounded wait of its kernels ran out)."""
+    _lib.check(_lib.load().whirgpu_rs_encode_status(ctx.handle), ctx.handle)
