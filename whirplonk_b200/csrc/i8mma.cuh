@@ -44,6 +44,19 @@ __device__ __forceinline__ bool mbar_wait(u32 bar, u32 parity) {
     }
     return false;
 }
+// The producer of a ring of bulk copies, before it leaves: the copies of the last
+// `armed` stages filled (the next one would be stage s in phase ph) have landed, so
+// the CTA's shared memory outlives them even when the consumers gave up.  Behind
+// consumers that did not, it waits for nothing.
+__device__ __forceinline__ bool ring_drain(u32 full, u32 stages, u32 s, u32 ph, u32 armed) {
+    bool ok = true;
+    for (; armed > 0; --armed) {
+        if (s == 0) s = stages, ph ^= 1;
+        --s;
+        ok = mbar_wait(full + 8 * s, ph) && ok;
+    }
+    return ok;
+}
 
 // K-major shared-memory operand, rows of 128 bytes in 8-row atoms of 1024
 // bytes, 128-byte swizzle (16-byte chunk c of row r at chunk c ^ (r mod 8)).

@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(32 * (CG_EPI_WARPS + 2), 1) k_cov_gemm(const _
                              "l"(src), "r"(bytes), "r"(bar)
                              : "memory");
             };
-            u32 s = 0, ph = 0;
-            for (u32 c = 0; c < a.chunks && ok; ++c) {
+            u32 s = 0, ph = 0, armed = 0;
+            for (u32 c = 0; c < a.chunks; ++c) {
                 ok = mbar_wait(empty + 8 * s, ph ^ 1);
                 if (!ok) break;
                 const u32 bytes = (two ? 4 : 3) * BLK;
@@ -138,13 +138,15 @@ __global__ void __launch_bounds__(32 * (CG_EPI_WARPS + 2), 1) k_cov_gemm(const _
                 copy(st, a.A + ((u64)mt * a.chunks + c) * BLK, BLK, full + 8 * s);
                 if (two) copy(st + BLK, a.A + ((u64)(mt + 1) * a.chunks + c) * BLK, BLK, full + 8 * s);
                 copy(st + 2 * BLK, a.B + ((u64)blockIdx.x * a.chunks + c) * 2 * BLK, 2 * BLK, full + 8 * s);
+                armed = min(armed + 1, CG_STAGES);
                 if (++s == CG_STAGES) s = 0, ph ^= 1;
             }
+            ok = ring_drain(full, CG_STAGES, s, ph, armed) && ok;
         }
     } else if (warp == CG_EPI_WARPS + 1) {
         if (lane == 0) {
             u32 s = 0, ph = 0;
-            for (u32 c = 0; c < a.chunks && ok; ++c) {
+            for (u32 c = 0; c < a.chunks; ++c) {
                 ok = mbar_wait(full + 8 * s, ph);
                 if (!ok) break;
                 tc_after();
@@ -159,6 +161,7 @@ __global__ void __launch_bounds__(32 * (CG_EPI_WARPS + 2), 1) k_cov_gemm(const _
                 if (++s == CG_STAGES) s = 0, ph ^= 1;
             }
             mma_commit(done);
+            ok = mbar_wait(done, 0) && ok;  // the contractions end before their memory goes
         }
     } else {
         ok = mbar_wait(done, 0);

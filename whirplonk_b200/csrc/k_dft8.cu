@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(JT + 32, 1) k_dft8(const __grid_constant__ Dft
     constexpr int G1 = BATCH >> E1;
     extern __shared__ unsigned char smem_raw[];
     __shared__ u32 s_tmem;
-    __shared__ __align__(8) u64 s_bar[4];
+    __shared__ __align__(8) u64 s_bar[5];
     const u32 base = (smem_u32(smem_raw) + 1023) & ~1023u;
     unsigned char* const gbase = smem_raw + (base - smem_u32(smem_raw));
     const u32 tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -306,6 +306,7 @@ __global__ void __launch_bounds__(JT + 32, 1) k_dft8(const __grid_constant__ Dft
     u64* const gT = reinterpret_cast<u64*>(gB + C::B1 + C::B2);
     const u32 smB1 = base + 2 * C::DATA, smB2 = smB1 + C::B1;
     const u32 full = smem_u32(&s_bar[0]), done = smem_u32(&s_bar[2]);  // [b] at + 8 b
+    const u32 drain = smem_u32(&s_bar[4]);
 
     if (issuer) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "n"(2 * REGION)
@@ -317,6 +318,7 @@ __global__ void __launch_bounds__(JT + 32, 1) k_dft8(const __grid_constant__ Dft
             mbar_init(full + 8 * b, WARPS);
             mbar_init(done + 8 * b, 1);
         }
+        mbar_init(drain, 1);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     tc_before();
@@ -559,10 +561,11 @@ __global__ void __launch_bounds__(JT + 32, 1) k_dft8(const __grid_constant__ Dft
         };
         last_round(std::integral_constant<int, E1>{}, b, C::HALVES == 2 ? b * (16 / C::HALVES) : 0, dest, before);
     };
-    // The issuer's contractions of region b.
+    // The issuer's contractions of region b (none after a wait that ran out: their
+    // operand may still be written).
     auto contract = [&](u32 b, u32 buf, bool second) {
         await(full, b);
-        if (lane != 0) return;
+        if (lane != 0 || !ok) return;
         const u32 smD = base + buf * C::DATA, d = tmem + b * REGION;
         constexpr int NO = 16 / C::HALVES;
         if (!second) {
@@ -679,8 +682,13 @@ __global__ void __launch_bounds__(JT + 32, 1) k_dft8(const __grid_constant__ Dft
     }
     if (!ok && a.err) atomicOr_system(a.err, TX_ERR_TIMEOUT);
     tc_before();
-    __syncthreads();
+    const bool failed = __syncthreads_or(!ok);
     if (issuer) {
+        if (failed && lane == 0) {  // the contractions under way end before their memory goes
+            mma_commit(drain);
+            mbar_wait(drain, 0);
+        }
+        __syncwarp();
         tc_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(2 * REGION));
     }
