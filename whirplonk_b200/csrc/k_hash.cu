@@ -592,7 +592,7 @@ int launch_merkle_batch(u32* nodes, u32 logN, u32 count, u64 node_stride, cudaSt
 // sums and sends the values as prover messages, point-major, every evaluated
 // vector at each point.
 // ---------------------------------------------------------------------------
-// OOD_GRID: capacity of the per-CTA partials (the grid is 4 CTAs per SM, at most this).
+// OOD_GRID: capacity of the per-CTA partials (k_ood's grid is 4 CTAs per SM, at most this).
 constexpr int OOD_GRID = 1024, OOD_THREADS = 256;
 constexpr u32 OOD_LO = 10;
 constexpr int OOD_MAX_VALUES = MAX_OOD * MAX_VECTORS;
@@ -677,9 +677,8 @@ __device__ __forceinline__ E3 ood_part(const OodArgs& a, const E3* zlo, const E3
 // bit.  Bound at small sizes by the chain of squarings and sums, at large ones by
 // the products.  Against a launch of its own for the tables (serial powers, up to
 // two products a bit) and every table entry read through L2, all values of a proof
-// on B200: n = 12 64 -> 47 us (3), n = 16 88 -> 68 (4), n = 18 94 -> 73 (4),
-// n = 20 127 -> 123 (5), n = 24 262 -> 238 (6).  Several values keep the table
-// launch: their powers are shared.
+// on B200: n = 12 64 -> 47 us (3), n = 16 88 -> 68 (4), n = 18 94 -> 73 (4); with
+// the PoW challenge that either draws since, n = 24 279 -> 231 (6).  Several values keep the table launch: their powers are shared.
 __global__ void __launch_bounds__(OOD_THREADS) k_ood_one(const __grid_constant__ OodArgs a, u32 len_log, u64 parts,
                                                          u32 squares, E3* partials, unsigned* counter) {
     __shared__ E3 zl[1u << OOD_LO];
@@ -858,12 +857,18 @@ int launch_ood(const OodArgs& a, cudaStream_t st) {
     const u64 warps_per_cta = OOD_THREADS / 32;
     const u64 cap = std::min<u64>(4ull * device_sms(), (u64)OOD_GRID);
     if (a.n_ood == 1 && a.nvec == 1 && a.skip_lo >= a.skip_hi) {
+        // Two CTAs an SM are resident (104 registers a thread), and every CTA forms
+        // its powers: a second wave of CTAs would form them again.  Four CTAs an SM
+        // took n = 24 from 231 to 259 us (all values of a proof), n = 20 from 121 to
+        // 133, and 24 mixed requests served together from 13.6 to 13.8 ms; one an SM
+        // takes n = 24 to 267.
+        const u64 most = std::min<u64>(2ull * device_sms(), (u64)OOD_GRID);
         // Parts of 2^10 coefficients, of fewer (down to 2^7) while they still fit
         // the grid's warps once.
         u32 len_log = OOD_LO;
-        while (len_log > OOD_LO - 3 && (a.size >> (len_log - 1)) <= cap * warps_per_cta) --len_log;
+        while (len_log > OOD_LO - 3 && (a.size >> (len_log - 1)) <= most * warps_per_cta) --len_log;
         const u64 parts = (a.size + (1ull << len_log) - 1) >> len_log;
-        const u64 grid = std::min<u64>(cap, (parts + warps_per_cta - 1) / warps_per_cta);
+        const u64 grid = std::min<u64>(most, (parts + warps_per_cta - 1) / warps_per_cta);
         const u64 top = parts > grid * warps_per_cta ? grid * warps_per_cta : parts - 1;  // the largest factor's exponent / len
         u32 bits = 0;
         while (top >> bits) ++bits;
