@@ -303,7 +303,8 @@ __global__ void k_sc_after_pow(TxState* tx, ProofScalars* sc, int r_slot) {
 // ---------------------------------------------------------------------------
 constexpr u64 SC_SMALL_MAX = 1ull << 15;
 constexpr int SC_CL = 8;                // CTAs of a cluster
-constexpr u64 SC_CL_MIN = 1ull << 9;  // fewer elements: one CTA
+constexpr u64 SC_CL_MIN = 1ull << 9;    // fewer elements: one CTA
+constexpr u64 SC_ONE_MAX = 1ull << 12;  // the most that one CTA holds (192 KB)
 constexpr int SC_CL_THREADS = 256;   // folding threads of a CTA; one more warp for the transcript
 
 struct ScClusterArgs {
@@ -461,7 +462,7 @@ __global__ void __launch_bounds__(SC_CL_THREADS + 32, 1) k_sumcheck_cluster(cons
 }
 
 static int sumcheck_cluster_prepare() {
-    const size_t cl = SC_SMALL_MAX / SC_CL * 48, one = SC_CL_MIN * 48;
+    const size_t cl = SC_SMALL_MAX / SC_CL * 48, one = SC_ONE_MAX * 48;
     return cudaFuncSetAttribute(k_sumcheck_cluster<SC_CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cl) == cudaSuccess &&
                    cudaFuncSetAttribute(k_sumcheck_cluster<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)one) == cudaSuccess
                ? 0
@@ -471,9 +472,12 @@ static int sumcheck_cluster_prepare() {
 int launch_sumcheck_small(const SumcheckArgs& s, int rounds, int fold_after, cudaStream_t st) {
     if (s.size > SC_SMALL_MAX || s.pow_threshold != ~0ull || rounds < 1) return 1;  // not this path
     if ((s.size >> rounds) < 1) return -1;
-    // The last round's halves still split over the cluster.
+    // A cluster while the last round's halves still split over it: a vector folded
+    // to fewer elements (the final sumcheck of a long final vector) takes one CTA.
+    // (Against a launch a round, whole prove calls on B200: 2^9 folded to one element
+    // 512 -> 450 us, 2^12 2686 -> 2635.)
     const bool cluster = s.size >= SC_CL_MIN && (s.size >> rounds) >= (u64)SC_CL;
-    if (!cluster && s.size >= SC_CL_MIN) return 1;
+    if (!cluster && s.size > SC_ONE_MAX) return 1;
     ScClusterArgs a{};
     a.a_base = s.a_base;
     for (int c = 0; c < 3; ++c) { a.a[c] = s.a_in[c]; a.b[c] = s.b[c]; }
