@@ -353,7 +353,14 @@ whirgpu_status whirgpu_rs_commit_batch(whirgpu_ctx* ctx, const uint64_t* vectors
                                        uint32_t log_len, uint32_t log_expansion, uint32_t log_depth, uint8_t* roots);
 
 /* ---- NTT pass plans (autotuned) ------------------------------------------------- */
-/* The LDE of a 2^log_n codeword from a 2^(log_n - log_expansion) message runs in
+/* Plans rule the encoder's butterfly passes.  From 2^20 codeword words (all planes
+ * together) up, messages of 2^8 .. 2^20 words run as two passes of 8-bit
+ * contractions instead, which have no plan: there only a plan given to
+ * whirgpu_ntt_set_plan takes the butterfly passes; autotuned, loaded and
+ * default plans apply to the other shapes and buffers (smaller ones, other message
+ * lengths, buffers that do not start at 16 bytes).
+ *
+ * The LDE of a 2^log_n codeword from a 2^(log_n - log_expansion) message runs in
  * npass passes of radix 2^log_radix[s] (sum = log_n, each <= 11); pass s stages
  * 2^log_cols[s] columns per CTA (255 = built-in choice); the kernel variant's
  * registers are sized for min_blocks CTAs per SM (2..4, 0 = built-in);
@@ -369,13 +376,17 @@ typedef struct {
 } whirgpu_ntt_plan;
 /* Times every valid plan for the shape on `planes` synthetic planes (median of
  * `reps` runs each), checks each plan's codeword against the built-in plan's,
- * installs the fastest agreeing plan for (log_n, log_expansion) and returns it.
- * Returns WHIRGPU_E_DEVICE (after installing) if any plan disagreed. */
+ * installs the fastest agreeing plan for (log_n, log_expansion) and returns it
+ * (for the butterfly passes, see above; it removes the effect of an earlier
+ * whirgpu_ntt_set_plan for the shape).  Returns WHIRGPU_E_DEVICE (after installing) if any plan disagreed. */
 whirgpu_status whirgpu_ntt_autotune(whirgpu_ctx* ctx, uint32_t log_n, uint32_t log_expansion, uint32_t planes,
                                     uint32_t reps, whirgpu_ntt_plan* best, double* best_us, uint32_t* tried);
-/* Installs a plan (npass = 0 removes the shape's plan); process-wide. */
+/* Installs a plan (npass = 0 removes the shape's plan); process-wide.  The shape
+ * then runs as butterfly passes by this plan, whatever its size.  A saved plan
+ * file does not keep that: loaded again, the plan is one like the others. */
 whirgpu_status whirgpu_ntt_set_plan(const whirgpu_ntt_plan* plan);
-/* The plan the encoder uses for a shape (installed, else built-in). */
+/* The plan of a shape's butterfly passes (installed, else built-in); whether the
+ * encoder takes them depends on the planes and buffers of a call, see above. */
 whirgpu_status whirgpu_ntt_get_plan(uint32_t log_n, uint32_t log_expansion, whirgpu_ntt_plan* out);
 void whirgpu_ntt_clear_plans(void);
 /* Installed plans (returns the count; writes at most cap). */

@@ -1,7 +1,8 @@
 """The encoder's contraction passes where a CTA takes many tiles of one coset (the
 two buffers handed over and over, odd and even tile counts), where tiles of
-several cosets meet in a CTA, short messages with many cosets, and buffers that start between 16-byte boundaries (which take the
-butterfly passes): word for word against the oracle's codewords."""
+several cosets meet in a CTA, short messages with many cosets, and buffers that
+start between 16-byte boundaries (which take the butterfly passes): word for word
+against the oracle's codewords."""
 import numpy as np
 import pytest
 

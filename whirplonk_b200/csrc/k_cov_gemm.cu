@@ -17,6 +17,11 @@
 // second.  Measured on B200, all covector updates of a proof (tables included):
 // n = 24 rate 1/4 425 -> 152 us, n = 20 rate 1/8 100 -> 88, n = 18 rate 1/2 121
 // -> 70.
+//
+// The operand images lie in the workspace's LDE scratch, which is free between
+// commitments.  Where that is smaller -- folding 1 at rate 1/2: 190 words a row at
+// 2^15 elements want 2.75 MB, and there are 1.5 -- the update runs from tables
+// (k_cov_accumulate), as it does for vectors whose planes do not start at 16 bytes.
 #include <algorithm>
 
 #include "gl.cuh"

@@ -551,9 +551,11 @@ static int merkle_levels_h(u32* nodes, u32 logN, TxState* tx, ProofScalars* sc, 
         const u32 levels = (logN - level) < 9 ? (logN - level) : 9;
         const u32 ctas = 1u << (logN - level - levels);
         const int finish = (level + levels == logN) ? 1 : 0;
-        // From four CTAs a SM on the hashes of the wide levels fill the ALU pipe:
-        // 64 trees of 2^13 leaves take 189 us end to end this way, 199 us with
-        // the short chains.
+        // From four CTAs a SM on the hashes of the wide levels fill the ALU pipe.  Whole
+        // commitments (us), additions on the FMA pipe / short chains: 64 trees of 2^13
+        // leaves 181 / 191, 64 of 2^14 468 / 480, 256 of 2^11 208 / 214, 512 of 2^10
+        // 264 / 270, 20 of 2^16 367 / 371; below it no difference (32 of 2^13 127 / 127,
+        // 128 of 2^11 129 / 129), and a tree alone is a chain.
         auto* const k = (u64)ctas * count >= 4ull * device_sms() ? k_merkle<H, true> : k_merkle<H, false>;
         k<<<dim3(ctas, count), 256, 0, st>>>(nodes, logN, level, levels, tx, sc, commit_idx, n_ood, finish, node_stride);
         count_launches(1);
