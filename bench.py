@@ -83,7 +83,7 @@ DEFAULT_WORKLOAD = "whir_served_mixed_n12_24"
 FALLBACK_HBM_GBS = 6650.0
 # Families whose kernels saturate the integer-ALU pipe before HBM (ncu summaries
 # in profiles/): their HBM fraction is low by nature.
-ALU_BOUND = {"ntt": "integer ALU pipe (67-76 % busy in ncu; butterflies of Goldilocks arithmetic)",
+ALU_BOUND = {"ntt": "integer ALU pipe (63-65 % busy in ncu: joins of the 8-bit contractions; butterflies below 2^20 words)",
              "leaf_hash": "integer ALU pipe (80-90 % busy in ncu; BLAKE3 compressions)",
              "merkle": "integer ALU pipe (BLAKE3 compressions)"}
 DATA = "synthetic (seeded ChaCha20 coefficients, seeded Ext3 points)"

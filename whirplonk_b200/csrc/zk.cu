@@ -621,13 +621,13 @@ whirgpu_status whirgpu_zk_commit(whirgpu_ctx* c, const whirgpu_zk_config* cfg, c
         return zk_fail(c, s, m);
     };
     // Counters and tickets of both workspaces start at zero (they reset themselves
-    // after use, as in the workspace cache): those in the scratch regions and the
-    // ProofScalars' (the transcript's start clears them in one workspace only, and
-    // the two proofs share one transcript).
-    auto clear_tickets = [&](const ProofPlan& p, char* ws) -> cudaError_t {
-        const cudaError_t e1 = cudaMemsetAsync(ws + p.off_sc_scratch, 0, p.off_tx - p.off_sc_scratch, c->stream);
-        if (e1 != cudaSuccess) return e1;
-        return cudaMemsetAsync(plan_scalars(p, ws)->counters, 0, sizeof(ProofScalars::counters), c->stream);
+    // after use, as in the workspace cache): those in the scratch regions and, behind
+    // them, the ProofScalars' (the transcript's start clears them in one workspace
+    // only, and the two proofs share one transcript).
+    auto clear_tickets = [&](const ProofPlan& p, char* ws) {
+        char* const end = reinterpret_cast<char*>(plan_scalars(p, ws) + 1);
+        char* const begin = ws + p.off_sc_scratch;
+        return cudaMemsetAsync(begin, 0, (size_t)(end - begin), c->stream);
     };
     cudaError_t e = clear_tickets(w->pb, dev + w->off_b);
     if (e == cudaSuccess) e = clear_tickets(w->pg, dev + w->off_g);
