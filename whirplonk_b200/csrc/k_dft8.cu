@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(JT + 32, 1) k_dft8(const __grid_constant__ Dft
         fence_async();
         tc_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(full + 8 * b);
+        if (lane == 0 && ok) mbar_arrive(full + 8 * b);  // after a wait that ran out nothing is handed on
     };
 
     // ---- a tile's loads: word pairs adjacent in memory, one round ahead -------

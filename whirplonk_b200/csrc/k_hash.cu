@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(RING_ROWS + 32, RING_CTAS) k_leaves_ring(const
                 // does not say (under load from other kernels it overtook them).
                 fence_async();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(empty + 8 * s);
+                if (lane == 0 && ok) mbar_arrive(empty + 8 * s);  // (a stage not waited for stays as it is)
                 if (++s == RING_STAGES) s = 0, ph ^= 1;
                 const unsigned flags = (t == 0 ? B3_CHUNK_START : 0u) | (t + 1 == a.nblocks ? (B3_CHUNK_END | B3_ROOT) : 0u);
                 b3_compress(cv, m, flags);
